@@ -458,10 +458,9 @@ fi_status advance_t(fi_model *m, int niter) {
             Ptrs<T> out = m->ptrs<T>(true);
             out.eta = in.eta;
             out.eta_next = in.eta_next;
-            alignas(64) unsigned char maps[18][128];
+            alignas(64) unsigned char maps[11][128];
             for (int f = 0; f < kState; f++) std::memcpy(maps[f], m->parity ? m->map_alt[f] : m->map_base[f], 128);
             std::memcpy(maps[10], m->map_eta[m->eta_swapped ? 1 : 0], 128);
-            for (int f = 0; f < 7; f++) std::memcpy(maps[11 + f], m->parity ? m->tmap_alt[f] : m->tmap_base[f], 128);
             FI_CHECK_CUDA(launch_fused3d<T>(m->g, m->kp, in, out, maps, m->fused_variant, m->d_err, m->stream),
                           "fused sweep");
             m->parity ^= 1;
@@ -487,21 +486,17 @@ fi_status check_err_word(fi_model *m) {
 }
 
 // (re)encode the tensor maps of every buffer the fused sweep reads, for the
-// current variant's tile shape: full boxes of the eleven inputs and trimmed boxes
-// of the seven stresses, for both state buffers
+// current variant's tile shape, for both state buffers
 fi_status encode_maps(fi_model *m) {
     const int v = m->fused_variant, key = fused3d_variant_key(v), esz = (int)m->esz;
     if (key == m->maps_key) return FI_OK;
     for (int f = 0; f < kState; f++) {
-        if (!fused3d_encode_map(field_raw(m->base[f], m->esz), m->g, esz, v, f, false, m->map_base[f]) ||
-            !fused3d_encode_map(field_raw(m->alt[f], m->esz), m->g, esz, v, f, false, m->map_alt[f]))
-            return set_error("cuTensorMapEncodeTiled failed"), FI_ERR_CUDA;
-        if (f < 7 && (!fused3d_encode_map(field_raw(m->base[f], m->esz), m->g, esz, v, f, true, m->tmap_base[f]) ||
-                      !fused3d_encode_map(field_raw(m->alt[f], m->esz), m->g, esz, v, f, true, m->tmap_alt[f])))
+        if (!fused3d_encode_map(field_raw(m->base[f], m->esz), m->g, esz, v, f, m->map_base[f]) ||
+            !fused3d_encode_map(field_raw(m->alt[f], m->esz), m->g, esz, v, f, m->map_alt[f]))
             return set_error("cuTensorMapEncodeTiled failed"), FI_ERR_CUDA;
     }
-    if (!fused3d_encode_map(field_raw(m->base[FI_FIELD_ETA], m->esz), m->g, esz, v, 10, false, m->map_eta[0]) ||
-        !fused3d_encode_map(field_raw(m->base[FI_FIELD_ETA_NEXT], m->esz), m->g, esz, v, 10, false, m->map_eta[1]))
+    if (!fused3d_encode_map(field_raw(m->base[FI_FIELD_ETA], m->esz), m->g, esz, v, 10, m->map_eta[0]) ||
+        !fused3d_encode_map(field_raw(m->base[FI_FIELD_ETA_NEXT], m->esz), m->g, esz, v, 10, m->map_eta[1]))
         return set_error("cuTensorMapEncodeTiled failed"), FI_ERR_CUDA;
     m->maps_key = key;
     return FI_OK;
@@ -613,8 +608,6 @@ fi_status advance_half(fi_model *m, int dim, int part) {
         out.eta_next = in.eta_next;
         for (int f = 0; f < kState; f++) std::memcpy(m->pend_maps[f], m->parity ? m->map_alt[f] : m->map_base[f], 128);
         std::memcpy(m->pend_maps[10], m->map_eta[m->eta_swapped ? 1 : 0], 128);
-        for (int f = 0; f < 7; f++)
-            std::memcpy(m->pend_maps[11 + f], m->parity ? m->tmap_alt[f] : m->tmap_base[f], 128);
         static_assert(sizeof(Ptrs<T>) <= sizeof(m->pend_ptrs[0]), "pending pointers fit");
         std::memcpy(m->pend_ptrs[0], &in, sizeof(in));
         std::memcpy(m->pend_ptrs[1], &out, sizeof(out));
@@ -732,6 +725,7 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
         return fail(cuda_fail(cudaGetLastError(), "activity bytes"));
     cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream);
     if (m->path == FI_PATH_FUSED) {
+        m->fused_variant = fused3d_default_variant(g);
         fi_status es = encode_maps(m);
         if (es != FI_OK) return fail(es);
     }
@@ -1019,14 +1013,6 @@ static fi_status make_shadow(fi_model *m) {
             }
         }
 
-    if (s->path == FI_PATH_FUSED && fused3d_num_variants() > 4) {
-        s->fused_variant = 4;  // 32x16 tiles: the FP32 shape the autotuner prefers on the slab
-        fi_status es = encode_maps(s);
-        if (es != FI_OK) {
-            fi_model_destroy(s);
-            return es;
-        }
-    }
     if (cudaStreamSynchronize(s->stream) != cudaSuccess) {
         fi_model_destroy(s);
         return cuda_fail(cudaGetLastError(), "shadow sync");

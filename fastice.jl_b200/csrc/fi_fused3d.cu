@@ -6,47 +6,59 @@
 // kernels touch the state twice per iteration (33 array passes); this sweep
 // reads P, τ(6), V(3), η once and writes P, τ(6), V(3), η_next once (22 passes).
 //
-// Work decomposition.  A CTA owns a TX x TY column of grid positions (x, y) and a
-// block of z planes (TX = 32 or 64: one or two x positions per thread, 32·TY
-// threads).  It marches up in z.  For every plane s the tensor-memory
-// accelerator copies an (x, y) box of each of the eleven input fields (old P, τ,
-// V, η; V.z one plane higher) into shared-memory plane rings, one plane ahead of
-// the compute, signalled by an mbarrier.  The new stresses of plane s are
-// computed in place over the column (all seven components) and over a
-// one-position ring (only the components the velocity update reads there), the
-// stress boundary conditions are applied to the plane in shared memory, and V /
-// η_next of plane s-1 are updated from the stress planes s-2, s-1, s.
-// Neighbouring CTAs recompute each other's ring: no grid-wide synchronisation.
+// Work decomposition.  A CTA owns a TX x TY column of grid positions (x, y), one
+// thread each, and a block of z planes [kb, ke).  It marches up in z.  Step s
+// computes the new P, τxx, τyy, τzz, τxy of plane s and the new τxz, τyz of plane
+// s + 1 (their staggered position is the face between the two planes), then V and
+// η_next of plane s: everything V(s) reads is then at hand in the same step, so the
+// centre stresses live in two shared-memory slots and a z-block re-reads one plane
+// of its neighbour below and one above.  P, τzz and η of the plane below, which V.z
+// needs in the thread's own column only, stay in registers.  A step s = kb - 1
+// before the march provides them and τxz, τyz of plane kb.
 //
-// Boxes.  A CTA whose column touches an x or y boundary loads every field over the
-// column plus the whole one-position ring (the boundary fix-ups and ghost writes
-// reach all of it).  An interior CTA of a "trimmed" launch shape loads each
-// stress component only where the sweep reads it: the ring stresses the velocity
-// update needs are P and τxx left of the column, P and τyy below it, τxy and τxz
-// right of it, τxy and τyz above it (and τxy at the upper right corner); τzz needs
-// no ring at all.  V and η keep the full ring.  This cuts the DRAM sectors an
-// interior column reads per plane by about a sixth (the ring is re-read by the
-// neighbouring columns).
+// Loads.  The tensor-memory accelerator copies an (x, y) box of each input field
+// into shared-memory plane slots, one step ahead, signalled by an mbarrier.  Group g
+// holds V, η, τxz, τyz of plane g and P, τxx, τyy, τzz, τxy of plane g - 1.  V and η
+// come with a one-position ring on every side; a stress component comes only with
+// the ring sides the velocity update reads: P and τxx left of the column, P and τyy
+// below it, τxy and τxz right of it, τxy and τyz above it, τzz with none.  A group's
+// slots are refilled as soon as every warp has left the velocity update that read
+// them: the last warp to arrive (an atomic counter) issues the copies, so no warp
+// waits for another there and a step has one block barrier.
+//
+// The new stresses are computed in place in shared memory, over the column and over
+// the ring sides above (neighbouring CTAs recompute each other's ring: no grid-wide
+// synchronisation).
 //
 // Clusters.  A launch shape may group CTAs into thread-block clusters (2x2, ...)
-// purely for co-scheduling: cluster members start together on one GPC and march
-// through z at the same pace, so the ring rows one member reads are the rows its
-// neighbour reads at about the same time and the second read hits L2.  There is no
-// cross-CTA communication and no multicast; a CTA may leave the cluster at any time.
+// purely for co-scheduling.  There is no cross-CTA communication and no multicast;
+// a CTA may leave the cluster at any time.
+//
+// What bounds it.  At 511^3 FP64 DRAM: 1.11 times the field bytes are read (the rings;
+// 64-byte L2 promotion) and the launch takes 4.35 ms, 5.6 TB/s of traffic; FP32 2.7 ms, half
+// DRAM and half instruction issue (53 % active).  Three FP64 CTAs fit an SM (70 KB of slots,
+// 80 registers), 24 warps; a form with 37 slots, two barriers a step, the boundary values
+// applied in passes over the plane and two CTAs per SM took 5.45 and 3.46 ms on the same
+// box.  Small grids are bound by the latency of a step (2.5-3 us alone on an SM), hence
+// the short z-blocks of fused3d_default_variant: 127^3 with walls 240 -> 115 us, 47x33x29
+// 138 -> 11 us.
 //
 // Double buffering.  Stresses and velocities are read from `in` and written to
 // `out` (distinct buffers), so the pointwise in-place updates of the reference
 // are reproduced exactly.  With a no-FMA build the sweep matches the CPU oracle
 // bit for bit.
 //
-// Boundary conditions.  Stress BCs are applied per plane in the order x-faces,
-// y-faces, z-faces (a face of dim d spans all positions in the dims before d and
-// the field's interior in the dims after d), as the CPU oracle does.  Velocity
-// Dirichlet values are written at the boundary nodes; ghost values (Velocity BC
-// ghosts 2c - v, η_next Neumann copies, periodic images) are written by the
-// thread that computes the interior value they derive from.  Periodic x / y need
-// no stress fix-up: ghost-ring stresses follow from the wrapped ghosts of the
-// previous iteration.
+// Boundary conditions.  They are applied in registers by the thread that computes
+// the value: fixed shear stresses at boundary nodes replace the value (x, then y,
+// then z faces, a later dimension's value wins, as the CPU oracle applies them),
+// and the thread that computes a P or τ_dd next to a traction side also writes its
+// ghost 2c - v.  Velocity Dirichlet values are written at the boundary nodes; ghost
+// values (Velocity BC ghosts 2c - v, η_next Neumann copies, periodic images) are
+// written by the thread that computes the interior value they derive from.  Periodic
+// x / y need no stress fix-up: the ghost-layer stresses (the ring of the first
+// column, written back by its ring threads) follow from the wrapped ghosts of V and
+// η of the previous iteration.  Stress ghosts that no update or residual reads are
+// not maintained.
 //
 // Waits.  Every mbarrier wait is bounded (about one second of SM clock); on
 // expiry the CTA records FI_ERR_TIMEOUT in the model's error word, waits once
@@ -68,95 +80,95 @@ namespace fi {
 
 namespace {
 
-// Launch shapes: tile width and height, z-block depth, cluster shape (x, y) and
-// whether interior tiles load trimmed stress boxes.  (Issuing the copies of plane
-// s+1 after the stress barrier of step s instead, which saves the barrier closing
-// each step, measured 15-20 % slower at 511^3: the copies then lose half their
-// lead.  Z-blocks of 16 and 24 planes on 32x8 tiles measured 3 % slower and equal
-// to 32 planes at 511^3 in both precisions: shorter blocks refill their rings
-// more often.)  Shapes whose shared memory does not fit a CTA for a precision
-// are not offered for it.
+// Launch shapes: tile width and height, z-block depth, cluster shape (x, y).  The
+// trim flag only marks names: every shape loads the trimmed boxes.  Shapes whose
+// shared memory does not fit a CTA for a precision are not offered for it.
+// fused3d_default_variant picks a 32x8 shape by the grid; the others stay for the
+// autotuner (511^3 FP64 on one box: 32x8 tiles 4.37 ms, 32x16 5.45, 1x4 clusters 4.48;
+// FP32 2.72, 2.86, 2.86 and 64x8 2.98 ms).
 struct Variant {
     int tx, ty, zb, cx, cy, trim;
 };
-// Measured at 511^3 (CUDA events, 30 iterations per shape, one box): the 32x8 tiles
-// with z-blocks of 32 lead in both precisions; trimmed interior boxes (5.23 against
-// 5.09 ms in FP64), clusters (5.39-5.90 ms) and 64-wide FP32 tiles (4.51-9.5 against
-// 3.40 ms) are slower, and their DRAM reads per cell at 255^3 are within 5 % of the
-// plain shape's (the ring sectors they save were L2 hits already).  They stay in the
-// table so that the autotuner re-checks them on every device.
 constexpr Variant kVariants[] = {
     {32, 8, 32, 1, 1, 0},  {32, 8, 64, 1, 1, 0},  {32, 8, 128, 1, 1, 0}, {32, 4, 64, 1, 1, 0},
     {32, 16, 32, 1, 1, 0}, {32, 16, 64, 1, 1, 0}, {32, 16, 128, 1, 1, 0},
-    // trimmed interior boxes, clusters
     {32, 8, 32, 1, 1, 1},  {32, 8, 32, 1, 4, 1},  {32, 8, 32, 2, 2, 0},
-    // 64-wide tiles (two x positions per thread; FP32 only)
-    {64, 8, 32, 1, 1, 0},  {64, 8, 32, 1, 1, 1}};
+    {64, 8, 32, 1, 1, 0},  {64, 8, 32, 1, 1, 1},
+    // short z-blocks: grids too small to fill the GPU with long columns
+    {32, 8, 1, 1, 1, 0},   {32, 8, 2, 1, 1, 0},   {32, 8, 4, 1, 1, 0},   {32, 8, 8, 1, 1, 0},
+    {32, 8, 12, 1, 1, 0},  {32, 8, 16, 1, 1, 0},  {32, 8, 24, 1, 1, 0}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 // input fields in map order
 enum { M_P = 0, M_XX, M_YY, M_ZZ, M_XY, M_XZ, M_YZ, M_VX, M_VY, M_VZ, M_ET, M_COUNT };
-constexpr int kTrimmed = 7;  // fields with a trimmed box (the stresses)
 
-// shared-memory plane slots: ring base and length per field
-enum {
-    S_P = 0, R_P = 4,
-    S_ZZ = 4, R_ZZ = 4,
-    S_XX = 8, R_XX = 3,
-    S_YY = 11, R_YY = 3,
-    S_XY = 14, R_XY = 3,
-    S_XZ = 17, R_XZ = 3,
-    S_YZ = 20, R_YZ = 3,
-    S_VX = 23, R_VX = 3,
-    S_VY = 26, R_VY = 3,
-    S_VZ = 29, R_VZ = 4,
-    S_ET = 33, R_ET = 4,
-    S_COUNT = 37
-};
 constexpr int kBars = 3;
 constexpr int kSmemPerSM = 233472;  // bytes of shared memory per SM (228 KB)
 
-template <typename T, int TX, int TY>
-struct Layout {
-    // the box starts XB positions left of the column so that its global x
-    // coordinate times the element size is a multiple of 16 bytes
-    static constexpr int XB = 16 / (int)sizeof(T);
-    static constexpr int BX = ((TX + 1 + XB + XB - 1) / XB) * XB;  // full box width (column + ring, aligned)
-    static constexpr int RY = TY + 2;
-    static constexpr int PLANE = BX * RY;  // elements in one full box
-    static constexpr int PLANE_BYTES = PLANE * (int)sizeof(T);
-    static constexpr int SLOT = ((PLANE_BYTES + 127) / 128) * 128 / (int)sizeof(T);  // 128-byte aligned slots
-    static constexpr int NT = 32 * TY;
-    static constexpr int PX = TX / 32;  // x positions per thread
-    static constexpr size_t SMEM = (size_t)S_COUNT * SLOT * sizeof(T) + 128;
-    static constexpr int MINB_RAW = kSmemPerSM / (int)(SMEM + 1024);
-    static constexpr int MINB = MINB_RAW < 1 ? 1 : (MINB_RAW > 4 ? 4 : MINB_RAW);
-};
+// x positions a box starts left of the column so that its global x coordinate times
+// the element size is a multiple of 16 bytes
+template <typename T>
+constexpr int box_xb() { return 16 / (int)sizeof(T); }
 
-// Box of input field F relative to the column origin (i0, j0): x from i0 + ox,
-// width bw; y from j0 + oy, height bh.  Full boxes cover the ring on all sides;
-// trimmed boxes (stresses of interior CTAs) only the ring sides read there.
-template <typename T, int TX, int TY, bool TRIM, int F>
+// Box of input field F relative to the column origin (i0, j0): x from i0 + ox, width
+// bw; y from j0 + oy, height bh.  A plane's boxes lie together in shared memory: two
+// slots of the five centre stresses (P .. τxy), then three of the six face fields (τxz,
+// τyz, V, η); OFF is the box's element offset inside its slot (128-byte aligned).
+template <typename T, int TX, int TY, int F>
 struct FBox {
-    using L = Layout<T, TX, TY>;
-    static constexpr bool full = !TRIM || F >= kTrimmed;
-    static constexpr int ox = full ? -L::XB : ((F == M_P || F == M_XX) ? -L::XB : 0);
-    static constexpr int bw = full ? L::BX : ((F == M_ZZ || F == M_YY || F == M_YZ) ? TX : TX + L::XB);
-    static constexpr int oy = full ? -1 : ((F == M_P || F == M_YY) ? -1 : 0);
-    static constexpr int bh = full ? TY + 2 : ((F == M_XX || F == M_ZZ || F == M_XZ) ? TY : TY + 1);
+    static constexpr int XB = box_xb<T>();
+    static constexpr bool full = F >= M_VX;
+    static constexpr bool left = full || F == M_P || F == M_XX, right = full || F == M_XY || F == M_XZ;
+    static constexpr bool below = full || F == M_P || F == M_YY, above = full || F == M_XY || F == M_YZ;
+    static constexpr int ox = left ? -XB : 0;
+    static constexpr int bw = TX + (left ? XB : 0) + (right ? XB : 0);
+    static constexpr int oy = below ? -1 : 0;
+    static constexpr int bh = TY + (below ? 1 : 0) + (above ? 1 : 0);
     static constexpr int bytes = bw * bh * (int)sizeof(T);
-    static_assert(bw * bh <= L::SLOT, "box fits its slot");
+    static constexpr int elems = ((bytes + 127) / 128) * 128 / (int)sizeof(T);
+    static constexpr int off() {
+        if constexpr (F == M_P || F == M_XZ) return 0;
+        else return FBox<T, TX, TY, F - 1>::off() + FBox<T, TX, TY, F - 1>::elems;
+    }
+    static constexpr int OFF = off();
     static_assert((bw * (int)sizeof(T)) % 16 == 0, "TMA box rows are whole 16-byte units");
 };
 
-// the input maps of one sweep: eleven full-box maps in map order, then the trimmed
-// maps of the seven stress fields (used by interior CTAs of trimmed shapes)
-struct InMaps {
-    CUtensorMap m[M_COUNT];
-    CUtensorMap t[kTrimmed];
+template <typename T, int TX, int TY>
+struct Layout {
+    static constexpr int NT = TX * TY;
+    static constexpr int NW = NT / 32;
+    static constexpr int CS = FBox<T, TX, TY, M_XY>::OFF + FBox<T, TX, TY, M_XY>::elems;  // a slot of centre stresses
+    static constexpr int VS = FBox<T, TX, TY, M_ET>::OFF + FBox<T, TX, TY, M_ET>::elems;  // a slot of face fields
+    static constexpr int ELEMS = 2 * CS + 3 * VS;
+    static constexpr size_t SMEM = (size_t)ELEMS * sizeof(T) + 64;  // + mbarriers and the release counter
+    static constexpr int FIT = kSmemPerSM / (int)(SMEM + 1024);
+    // resident CTAs asked of the compiler: as many as the shared memory holds, up to
+    // 24 warps (80 registers a thread) in FP64 and 32 (64 registers) in FP32
+    static constexpr int WANT = (sizeof(T) == 8 ? 768 : 1024) / NT;
+    static constexpr int MINB = FIT < 1 ? 1 : (WANT < 1 ? 1 : (FIT < WANT ? FIT : WANT));
 };
 
-template <typename T, int TX, int TY, bool TRIM>
+// the input maps of one sweep, in map order
+struct InMaps {
+    CUtensorMap m[M_COUNT];
+};
+
+// What a boundary column's thread has to do beyond the update, from its position alone
+// (computed once per march).
+enum ColFlag : unsigned {
+    CF_IN = 1u << 0,                                           // inside the vertex range
+    CF_CX = 1u << 1, CF_CY = 1u << 2,                          // centre stresses exist along x / y
+    CF_X0 = 1u << 3, CF_X1 = 1u << 4, CF_Y0 = 1u << 5, CF_Y1 = 1u << 6,      // fixed shear nodes
+    CF_TX0 = 1u << 7, CF_TX1 = 1u << 8, CF_TY0 = 1u << 9, CF_TY1 = 1u << 10, // traction ghosts beside
+    CF_VX0 = 1u << 11, CF_VX1 = 1u << 12, CF_VY0 = 1u << 13, CF_VY1 = 1u << 14,  // fixed velocity nodes
+    CF_ONX = 1u << 15, CF_ONY = 1u << 16, CF_ONC = 1u << 17,   // V.x / V.y / V.z and η exist here
+    CF_IMG = 1u << 18,                                         // values here have images
+    CF_DUP = 1u << 19                                          // some have two along one dimension
+};
+constexpr unsigned CF_SHEAR = CF_X0 | CF_X1 | CF_Y0 | CF_Y1, CF_TRAC = CF_TX0 | CF_TX1 | CF_TY0 | CF_TY1;
+
+template <typename T, int TX, int TY>
 struct Ctx {
     using Lay = Layout<T, TX, TY>;
     T *sm;
@@ -166,595 +178,638 @@ struct Ctx {
     // the ghost layer on the low / high side of x / y comes from elsewhere: a periodic
     // image, or a neighbouring subdomain's halo (FI_BC_PERIODIC / FI_BC_HALO)
     bool hx0, hx1, hy0, hy1;
-    bool bnd_x, bnd_y;  // column touches an x / y boundary (needs fix-ups or ghost writes)
-    // Ring positions relative to the plane step sref: element offsets of the
-    // planes around sref inside three- and four-slot rings, computed once per plane
-    // step.  Every access names its plane as sref plus a constant, so after
-    // inlining the choice folds to one register (no modulo per access).
-    int sref;
-    int o3m, o30, o3p;                 // three-slot rings: planes sref-1, sref, sref+1
-    int o4m2, o4m, o40, o4p, o4p2;     // four-slot rings: planes sref-2 .. sref+2
+    // byte offsets of the slots of the step's planes: centre stresses of plane s, face
+    // fields of s and s + 1
+    unsigned C, V0, V1;
 
     __device__ __forceinline__ void set_plane(int s) {
-        sref = s;
-        const int m3 = s % 3, m4 = s & 3;
-        o30 = m3 * Lay::SLOT;
-        o3p = (m3 == 2 ? 0 : m3 + 1) * Lay::SLOT;
-        o3m = (m3 == 0 ? 2 : m3 - 1) * Lay::SLOT;
-        o4m2 = ((m4 + 2) & 3) * Lay::SLOT;
-        o4m = ((m4 + 3) & 3) * Lay::SLOT;
-        o40 = m4 * Lay::SLOT;
-        o4p = ((m4 + 1) & 3) * Lay::SLOT;
-        o4p2 = o4m2;
+        const unsigned p0 = (unsigned)s % 3u, p1 = p0 == 2u ? 0u : p0 + 1u;
+        C = (s & 1) * (unsigned)(Lay::CS * sizeof(T));
+        V0 = (unsigned)(2 * Lay::CS * sizeof(T)) + p0 * (unsigned)(Lay::VS * sizeof(T));
+        V1 = (unsigned)(2 * Lay::CS * sizeof(T)) + p1 * (unsigned)(Lay::VS * sizeof(T));
     }
-    // element index of (i, j) inside field F's box
-    template <int F>
-    __device__ __forceinline__ int ix(int i, int j) const {
-        using B = FBox<T, TX, TY, TRIM, F>;
-        return (j - j0 - B::oy) * B::bw + (i - i0 - B::ox);
-    }
-    template <int F>
-    __device__ __forceinline__ bool in_box(int i, int j) const {
-        using B = FBox<T, TX, TY, TRIM, F>;
-        const int a = i - i0 - B::ox, b = j - j0 - B::oy;
-        return a >= 0 && a < B::bw && b >= 0 && b < B::bh;
-    }
-    __device__ __forceinline__ T *slot(int base, int len, int p) const {
-        const int d = p - sref;
-        const int off = len == 3 ? (d < 0 ? o3m : d == 0 ? o30 : o3p)
-                                 : (d < -1 ? o4m2 : d == -1 ? o4m : d == 0 ? o40 : d == 1 ? o4p : o4p2);
-        return sm + base * Lay::SLOT + off;
-    }
-    __device__ __forceinline__ T &P(int p, int i, int j) const { return slot(S_P, R_P, p)[ix<M_P>(i, j)]; }
-    __device__ __forceinline__ T &Tzz(int p, int i, int j) const { return slot(S_ZZ, R_ZZ, p)[ix<M_ZZ>(i, j)]; }
-    __device__ __forceinline__ T &Txx(int p, int i, int j) const { return slot(S_XX, R_XX, p)[ix<M_XX>(i, j)]; }
-    __device__ __forceinline__ T &Tyy(int p, int i, int j) const { return slot(S_YY, R_YY, p)[ix<M_YY>(i, j)]; }
-    __device__ __forceinline__ T &Txy(int p, int i, int j) const { return slot(S_XY, R_XY, p)[ix<M_XY>(i, j)]; }
-    __device__ __forceinline__ T &Txz(int p, int i, int j) const { return slot(S_XZ, R_XZ, p)[ix<M_XZ>(i, j)]; }
-    __device__ __forceinline__ T &Tyz(int p, int i, int j) const { return slot(S_YZ, R_YZ, p)[ix<M_YZ>(i, j)]; }
-    __device__ __forceinline__ T Vx(int p, int i, int j) const { return slot(S_VX, R_VX, p)[ix<M_VX>(i, j)]; }
-    __device__ __forceinline__ T Vy(int p, int i, int j) const { return slot(S_VY, R_VY, p)[ix<M_VY>(i, j)]; }
-    __device__ __forceinline__ T Vz(int p, int i, int j) const { return slot(S_VZ, R_VZ, p)[ix<M_VZ>(i, j)]; }
-    __device__ __forceinline__ T Eta(int p, int i, int j) const { return slot(S_ET, R_ET, p)[ix<M_ET>(i, j)]; }
-    __device__ __forceinline__ long long gidx(int i, int j, int k) const {
-        return (long long)i + sx * (long long)j + sxy * (long long)k;
-    }
-    __device__ __forceinline__ bool own_x(int i) const {
-        if (i >= 1 && i <= n0 + 1) return i >= i0 && i < i0 + TX;
-        if (i == 0) return i0 == 1;
-        return i == n0 + 2 && n0 + 1 < i0 + TX;
-    }
-    __device__ __forceinline__ bool own_y(int j) const {
-        if (j >= 1 && j <= n1 + 1) return j >= j0 && j < j0 + TY;
-        if (j == 0) return j0 == 1;
-        return j == n1 + 2 && n1 + 1 < j0 + TY;
+    __device__ __forceinline__ unsigned col(int li, int lj) const {
+        return (unsigned)(i0 + li) + (unsigned)sx * (unsigned)(j0 + lj);
     }
 };
+
+// element of field F at the position (li, lj) from the column origin, in the slot at a
+// byte offset: the boxes have three row pitches, so a step's addresses are a few byte
+// offsets per thread plus constants
+template <int F, int TX, int TY, typename T>
+__device__ __forceinline__ T *el(unsigned slot, int li, int lj) {
+    using B = FBox<T, TX, TY, F>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    constexpr int K = (B::OFF - (B::oy * B::bw + B::ox)) * (int)sizeof(T);
+    return reinterpret_cast<T *>(smem_raw + (slot + (unsigned)((lj * B::bw + li) * (int)sizeof(T))) + K);
+}
+#define EL(F, slot) (el<F, TX, TY, T>(slot, li, lj))
 
 template <typename T>
 __device__ __forceinline__ T h(T x) { return T(0.5) * x; }
 
-// one box copy of field F of plane p into its ring slot
-template <int F, typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void load_box(const Ctx<T, TX, TY, TRIM> &c, const InMaps &mp, T *dst, int p, uint64_t *bar) {
-    using B = FBox<T, TX, TY, TRIM, F>;
-    const CUtensorMap *map = (TRIM && F < kTrimmed) ? &mp.t[F] : &mp.m[F];
-    tma_load_3d(dst, map, (int)kXOff + c.i0 + B::ox, c.j0 + B::oy, p, bar);
-}
-
-// issue the TMA copies of input group p (planes: σ_old(p), Vx(p), Vy(p), Vz(p+1), η(p))
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void issue_group(const Ctx<T, TX, TY, TRIM> &c, const InMaps &mp, int p, bool full,
-                                            uint64_t *bar) {
-    constexpr uint32_t vbytes = FBox<T, TX, TY, TRIM, M_VX>::bytes + FBox<T, TX, TY, TRIM, M_VY>::bytes +
-                                FBox<T, TX, TY, TRIM, M_VZ>::bytes + FBox<T, TX, TY, TRIM, M_ET>::bytes;
-    constexpr uint32_t sbytes = FBox<T, TX, TY, TRIM, M_P>::bytes + FBox<T, TX, TY, TRIM, M_XX>::bytes +
-                                FBox<T, TX, TY, TRIM, M_YY>::bytes + FBox<T, TX, TY, TRIM, M_ZZ>::bytes +
-                                FBox<T, TX, TY, TRIM, M_XY>::bytes + FBox<T, TX, TY, TRIM, M_XZ>::bytes +
-                                FBox<T, TX, TY, TRIM, M_YZ>::bytes;
-    mbar_expect_tx(bar, full ? vbytes + sbytes : vbytes);
-    if (full) {
-        load_box<M_P>(c, mp, c.slot(S_P, R_P, p), p, bar);
-        load_box<M_XX>(c, mp, c.slot(S_XX, R_XX, p), p, bar);
-        load_box<M_YY>(c, mp, c.slot(S_YY, R_YY, p), p, bar);
-        load_box<M_ZZ>(c, mp, c.slot(S_ZZ, R_ZZ, p), p, bar);
-        load_box<M_XY>(c, mp, c.slot(S_XY, R_XY, p), p, bar);
-        load_box<M_XZ>(c, mp, c.slot(S_XZ, R_XZ, p), p, bar);
-        load_box<M_YZ>(c, mp, c.slot(S_YZ, R_YZ, p), p, bar);
-    }
-    load_box<M_VX>(c, mp, c.slot(S_VX, R_VX, p), p, bar);
-    load_box<M_VY>(c, mp, c.slot(S_VY, R_VY, p), p, bar);
-    load_box<M_VZ>(c, mp, c.slot(S_VZ, R_VZ, p + 1), p + 1, bar);
-    load_box<M_ET>(c, mp, c.slot(S_ET, R_ET, p), p, bar);
-}
-
-// raw stress update of plane s at (i, j): which components is a compile-time mask.
-// Every shared-memory operand is loaded before the first store (the in-place stress
-// stores and the global writes go through pointers the compiler cannot separate from
-// the loads), so the seven updates form independent chains.  A component outside the
-// mask is neither loaded nor stored (a trimmed box may not hold it at (i, j)).
-enum { F_P = 1, F_XX = 2, F_YY = 4, F_ZZ = 8, F_XY = 16, F_XZ = 32, F_YZ = 64, F_ALL = 127 };
-
-// XYI: the column and its ring lie inside every x / y range (no boundary column),
-// so only the z ranges are tested
-template <typename T, int TX, int TY, bool TRIM, bool XYI>
-__device__ __forceinline__ void sigma_point(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q, int s,
-                                            int i, int j, int mask, bool write_now, const Ptrs<T> &out) {
-    if (!XYI && (i > c.n0 + 2 || j > c.n1 + 2)) return;
-    using Cx = Ctx<T, TX, TY, TRIM>;
-    constexpr int BV = FBox<T, TX, TY, TRIM, M_VX>::bw;  // row pitch of the V and η boxes
-    const T idx = q.inv_dx[0], idy = q.inv_dx[1], idz = q.inv_dx[2];
-    const bool cz = s >= 1 && s <= c.n2, vz = s >= 1 && s <= c.n2 + 1;
-    const bool cx = XYI || (i >= 1 && i <= c.n0) || (c.hx0 && i == 0) || (c.hx1 && i == c.n0 + 1);
-    const bool vx = XYI || (i >= 1 && i <= c.n0 + 1);
-    const bool cy = XYI || (j >= 1 && j <= c.n1) || (c.hy0 && j == 0) || (c.hy1 && j == c.n1 + 1);
-    const bool vy = XYI || (j >= 1 && j <= c.n1 + 1);
-    const int a = c.template ix<M_VX>(i, j);
-    const T *vxs = c.slot(S_VX, R_VX, s), *vys = c.slot(S_VY, R_VY, s), *vzs = c.slot(S_VZ, R_VZ, s);
-    const T *vxm = c.slot(S_VX, R_VX, s - 1), *vym = c.slot(S_VY, R_VY, s - 1), *vzp = c.slot(S_VZ, R_VZ, s + 1);
-    const T *et = c.slot(S_ET, R_ET, s), *etm = c.slot(S_ET, R_ET, s - 1);
-    T *sP = c.slot(S_P, R_P, s) + c.template ix<M_P>(i, j);
-    T *sXX = c.slot(S_XX, R_XX, s) + c.template ix<M_XX>(i, j);
-    T *sYY = c.slot(S_YY, R_YY, s) + c.template ix<M_YY>(i, j);
-    T *sZZ = c.slot(S_ZZ, R_ZZ, s) + c.template ix<M_ZZ>(i, j);
-    T *sXY = c.slot(S_XY, R_XY, s) + c.template ix<M_XY>(i, j);
-    T *sXZ = c.slot(S_XZ, R_XZ, s) + c.template ix<M_XZ>(i, j);
-    T *sYZ = c.slot(S_YZ, R_YZ, s) + c.template ix<M_YZ>(i, j);
-    (void)sizeof(Cx);
-    const bool dc = (mask & (F_P | F_XX | F_YY | F_ZZ)) && cx && cy && cz;
-    const bool dxy = (mask & F_XY) && vx && vy && cz;
-    const bool dxz = (mask & F_XZ) && vx && cy && vz;
-    const bool dyz = (mask & F_YZ) && cx && vy && vz;
-    // old values (all seven when the point is written out)
-    const int lmask = write_now ? F_ALL : mask;
-    T oP = T(0), oXX = T(0), oYY = T(0), oZZ = T(0), oXY = T(0), oXZ = T(0), oYZ = T(0);
-    if (lmask & F_P) oP = *sP;
-    if (lmask & F_XX) oXX = *sXX;
-    if (lmask & F_YY) oYY = *sYY;
-    if (lmask & F_ZZ) oZZ = *sZZ;
-    if (lmask & F_XY) oXY = *sXY;
-    if (lmask & F_XZ) oXZ = *sXZ;
-    if (lmask & F_YZ) oYZ = *sYZ;
-    T nP = oP, nXX = oXX, nYY = oYY, nZZ = oZZ, nXY = oXY, nXZ = oXZ, nYZ = oYZ;
-    if (dc) {
-        T exx = (vxs[a + 1] - vxs[a]) * idx;
-        T eyy = (vys[a + BV] - vys[a]) * idy;
-        T ezz = (vzp[a] - vzs[a]) * idz;
-        T divV = exx + eyy + ezz;
-        T etac = et[a];
-        if (mask & F_P) nP = oP - (p.p_forcing ? divV + __ldg(out.fP + c.gidx(i, j, s)) : divV) * etac * q.dt_P;
-        if (mask & F_XX) nXX = oXX - (oXX - T(2.0) * etac * (exx - third(divV))) * q.dt_tau[0];
-        if (mask & F_YY) nYY = oYY - (oYY - T(2.0) * etac * (eyy - third(divV))) * q.dt_tau[1];
-        if (mask & F_ZZ) nZZ = oZZ - (oZZ - T(2.0) * etac * (ezz - third(divV))) * q.dt_tau[2];
-    }
-    if (dxy) {
-        T exy = T(0.5) * ((vys[a] - vys[a - 1]) * idx + (vxs[a] - vxs[a - BV]) * idy);
-        T e_xy = h(h(et[a - 1 - BV] + et[a - BV]) + h(et[a - 1] + et[a]));
-        nXY = oXY - (oXY - T(2.0) * e_xy * exy) * q.dt_tau[3];
-    }
-    if (dxz) {
-        T exz = T(0.5) * ((vzs[a] - vzs[a - 1]) * idx + (vxs[a] - vxm[a]) * idz);
-        T e_xz = h(h(etm[a - 1] + etm[a]) + h(et[a - 1] + et[a]));
-        nXZ = oXZ - (oXZ - T(2.0) * e_xz * exz) * q.dt_tau[4];
-    }
-    if (dyz) {
-        T eyz = T(0.5) * ((vzs[a] - vzs[a - BV]) * idy + (vys[a] - vym[a]) * idz);
-        T e_yz = h(h(etm[a - BV] + etm[a]) + h(et[a - BV] + et[a]));
-        nYZ = oYZ - (oYZ - T(2.0) * e_yz * eyz) * q.dt_tau[5];
-    }
-    if (dc) {
-        if (mask & F_P) *sP = nP;
-        if (mask & F_XX) *sXX = nXX;
-        if (mask & F_YY) *sYY = nYY;
-        if (mask & F_ZZ) *sZZ = nZZ;
-    }
-    if (dxy) *sXY = nXY;
-    if (dxz) *sXZ = nXZ;
-    if (dyz) *sYZ = nYZ;
-    if (write_now) {
-        const long long I = c.gidx(i, j, s);
-        out.P[I] = nP;
-        out.txx[I] = nXX;
-        out.tyy[I] = nYY;
-        out.tzz[I] = nZZ;
-        out.txy[I] = nXY;
-        out.txz[I] = nXZ;
-        out.tyz[I] = nYZ;
-    }
-}
-
-// ring stresses of plane s (see sigma_plane); a warp spans a row of 32 positions
-// (TX / 32 per lane), TY < 32
-template <typename T, int TX, int TY, bool TRIM, bool XYI>
-__device__ __forceinline__ void sigma_ring(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q, int s,
-                                           const Ptrs<T> &out) {
-    constexpr int NW = Layout<T, TX, TY>::NT / 32;
-    constexpr int PX = TX / 32;
-    static_assert(TY < 32 && NW >= 4, "one ring side per warp");
-    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (w == NW - 4) {
-#pragma unroll
-        for (int u = 0; u < PX; u++)
-            sigma_point<T, TX, TY, TRIM, XYI>(c, p, q, s, c.i0 + lane + 32 * u, c.j0 - 1, F_P | F_YY, false, out);
-    } else if (w == NW - 3) {
-#pragma unroll
-        for (int u = 0; u < PX; u++)
-            sigma_point<T, TX, TY, TRIM, XYI>(c, p, q, s, c.i0 + lane + 32 * u, c.j0 + TY, F_XY | F_YZ, false, out);
-    } else if (w == NW - 2) {
-        if (lane < TY) sigma_point<T, TX, TY, TRIM, XYI>(c, p, q, s, c.i0 - 1, c.j0 + lane, F_P | F_XX, false, out);
-    } else if (w == NW - 1) {
-        if (lane < TY) sigma_point<T, TX, TY, TRIM, XYI>(c, p, q, s, c.i0 + TX, c.j0 + lane, F_XY | F_XZ, false, out);
-        else if (lane == TY) sigma_point<T, TX, TY, TRIM, XYI>(c, p, q, s, c.i0 + TX, c.j0 + TY, F_XY, false, out);
-    }
-}
-
-// stress boundary fix-ups of one face side on plane s at region point (i, j)
-// (boundary columns only: full boxes)
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void fix_x(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q, int s, int i,
-                                      int j, int side) {
-    const int kind = p.bc_kind[0][side];
-    if (kind != FI_BC_TRACTION && kind != FI_BC_SLIP) return;
-    const bool cz = s >= 1 && s <= c.n2, vz = s >= 1 && s <= c.n2 + 1;
-    const int ghost = side == 0 ? 0 : c.n0 + 1, adj = side == 0 ? 1 : c.n0, node = side == 0 ? 1 : c.n0 + 1;
-    if (kind == FI_BC_TRACTION && i == ghost && j >= 1 && j <= c.n1 && cz && adj >= c.i0 - 1 && adj <= c.i0 + TX) {
-        T tv = T(2.0) * q.bc_val[0][side][0];
-        c.P(s, i, j) = tv - c.P(s, adj, j);
-        c.Txx(s, i, j) = tv - c.Txx(s, adj, j);
-    }
-    if (i == node) {
-        if (j >= 1 && j <= c.n1 + 1 && cz) c.Txy(s, i, j) = q.bc_val[0][side][1];
-        if (j >= 1 && j <= c.n1 && vz) c.Txz(s, i, j) = q.bc_val[0][side][2];
-    }
-}
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void fix_y(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q, int s, int i,
-                                      int j, int side) {
-    const int kind = p.bc_kind[1][side];
-    if (kind != FI_BC_TRACTION && kind != FI_BC_SLIP) return;
-    const bool cz = s >= 1 && s <= c.n2, vz = s >= 1 && s <= c.n2 + 1;
-    const int ghost = side == 0 ? 0 : c.n1 + 1, adj = side == 0 ? 1 : c.n1, node = side == 0 ? 1 : c.n1 + 1;
-    if (kind == FI_BC_TRACTION && j == ghost && cz && adj >= c.j0 - 1 && adj <= c.j0 + TY) {
-        T tv = T(2.0) * q.bc_val[1][side][1];
-        c.P(s, i, j) = tv - c.P(s, i, adj);
-        c.Tyy(s, i, j) = tv - c.Tyy(s, i, adj);
-    }
-    if (j == node) {
-        if (cz) c.Txy(s, i, j) = q.bc_val[1][side][0];
-        if (vz) c.Tyz(s, i, j) = q.bc_val[1][side][2];
-    }
-}
-
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void sigma_plane(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q,
-                                            const Ptrs<T> &out, int s) {
+// issue the copies of group g: V, η of plane g; from kind 1 on the face stresses of
+// plane g and P, τzz of plane g - 1; kind 2: all centre stresses of plane g - 1
+template <typename T, int TX, int TY>
+__device__ __forceinline__ void issue_group(const Ctx<T, TX, TY> &c, const InMaps &mp, int g, int kind, uint64_t *bars) {
     using Lay = Layout<T, TX, TY>;
-    using Cx = Ctx<T, TX, TY, TRIM>;
-    constexpr int PX = Lay::PX;
-    const int tid = threadIdx.x, lane = tid % 32, row = tid / 32;
-    const bool zb_plane = s == 1 || s == c.n2 + 1;
-    const bool late = c.bnd_x || c.bnd_y || zb_plane;
-    const bool own_s = s >= c.kb && s < c.ke;
-    // pass 1: the column, all components; pass 2: the ring, only the components read
-    // there, one ring side per warp on the last four warps (one per scheduler), so
-    // that every ring warp takes a single branch path: the row below (P, τyy), the
-    // row above (τxy, τyz), the column left (P, τxx), the column right (τxy, τxz)
-    // with the corner above it (τxy)
-    if (TRIM || (!c.bnd_x && !c.bnd_y)) {
-#pragma unroll
-        for (int u = 0; u < PX; u++)
-            sigma_point<T, TX, TY, TRIM, true>(c, p, q, s, c.i0 + lane + 32 * u, c.j0 + row, F_ALL, own_s && !late, out);
-        sigma_ring<T, TX, TY, TRIM, true>(c, p, q, s, out);
-    } else {
-#pragma unroll
-        for (int u = 0; u < PX; u++)
-            sigma_point<T, TX, TY, TRIM, false>(c, p, q, s, c.i0 + lane + 32 * u, c.j0 + row, F_ALL, own_s && !late,
-                                                out);
-        sigma_ring<T, TX, TY, TRIM, false>(c, p, q, s, out);
+    constexpr uint32_t vb = 4u * FBox<T, TX, TY, M_VX>::bytes;
+    constexpr uint32_t fb = FBox<T, TX, TY, M_XZ>::bytes + FBox<T, TX, TY, M_YZ>::bytes + FBox<T, TX, TY, M_P>::bytes +
+                            FBox<T, TX, TY, M_ZZ>::bytes;
+    constexpr uint32_t cb = FBox<T, TX, TY, M_XX>::bytes + FBox<T, TX, TY, M_YY>::bytes + FBox<T, TX, TY, M_XY>::bytes;
+    const int q = g % 3;
+    uint64_t *bar = &bars[q];
+    T *V = c.sm + 2 * Lay::CS + q * Lay::VS, *C = c.sm + ((g - 1) & 1) * Lay::CS;
+    mbar_expect_tx(bar, vb + (kind > 0 ? fb : 0u) + (kind > 1 ? cb : 0u));
+#define FI_LOAD(F, slot, plane)                                                                                  \
+    tma_load_3d(slot + FBox<T, TX, TY, F>::OFF, &mp.m[F], (int)kXOff + c.i0 + FBox<T, TX, TY, F>::ox, \
+                c.j0 + FBox<T, TX, TY, F>::oy, plane, bar)
+    FI_LOAD(M_VX, V, g);
+    FI_LOAD(M_VY, V, g);
+    FI_LOAD(M_VZ, V, g);
+    FI_LOAD(M_ET, V, g);
+    if (kind > 0) {
+        FI_LOAD(M_XZ, V, g);
+        FI_LOAD(M_YZ, V, g);
+        FI_LOAD(M_P, C, g - 1);
+        FI_LOAD(M_ZZ, C, g - 1);
     }
-    __syncthreads();
-    if (!late) return;
-    constexpr int NREG = (TX + 2) * (TY + 2);
-    if constexpr (!TRIM) {
-        if (c.bnd_x && !(c.hx0 && c.hx1)) {  // fix_x leaves periodic and halo sides alone
-            for (int r = tid; r < NREG; r += Lay::NT) {
-                const int i = c.i0 - 1 + r % (TX + 2), j = c.j0 - 1 + r / (TX + 2);
-                fix_x<T, TX, TY, TRIM>(c, p, q, s, i, j, 0);
-                fix_x<T, TX, TY, TRIM>(c, p, q, s, i, j, 1);
-            }
-            __syncthreads();
-        }
-        if (c.bnd_y && !(c.hy0 && c.hy1)) {
-            for (int r = tid; r < NREG; r += Lay::NT) {
-                const int i = c.i0 - 1 + r % (TX + 2), j = c.j0 - 1 + r / (TX + 2);
-                fix_y<T, TX, TY, TRIM>(c, p, q, s, i, j, 0);
-                fix_y<T, TX, TY, TRIM>(c, p, q, s, i, j, 1);
-            }
-            __syncthreads();
-        }
+    if (kind > 1) {
+        FI_LOAD(M_XX, C, g - 1);
+        FI_LOAD(M_YY, C, g - 1);
+        FI_LOAD(M_XY, C, g - 1);
     }
-    if (zb_plane) {
-        const int side = s == 1 ? 0 : 1;
-        const int kind = p.bc_kind[2][side];
-        if (kind == FI_BC_TRACTION || kind == FI_BC_SLIP) {
-            const T c0 = q.bc_val[2][side][0], c1 = q.bc_val[2][side][1], tv = T(2.0) * q.bc_val[2][side][2];
-            for (int r = tid; r < NREG; r += Lay::NT) {
-                const int i = c.i0 - 1 + r % (TX + 2), j = c.j0 - 1 + r / (TX + 2);
-                // a trimmed box holds a component only where the sweep reads it
-                if (kind == FI_BC_TRACTION) {
-                    if (side == 0) {  // s == 1: ghost plane 0 from plane 1
-                        if (c.template in_box<M_P>(i, j)) c.P(s - 1, i, j) = tv - c.P(s, i, j);
-                        if (c.template in_box<M_ZZ>(i, j)) c.Tzz(s - 1, i, j) = tv - c.Tzz(s, i, j);
-                    } else {
-                        if (c.template in_box<M_P>(i, j)) c.P(s, i, j) = tv - c.P(s - 1, i, j);
-                        if (c.template in_box<M_ZZ>(i, j)) c.Tzz(s, i, j) = tv - c.Tzz(s - 1, i, j);
-                    }
-                }
-                if (c.template in_box<M_XZ>(i, j)) c.Txz(s, i, j) = c0;
-                if (c.template in_box<M_YZ>(i, j)) c.Tyz(s, i, j) = c1;
-            }
-            __syncthreads();
-        }
-    }
-    (void)sizeof(Cx);
-    const bool own_0 = s == 1 && c.kb == 1 && p.bc_kind[2][0] == FI_BC_TRACTION;
-    if (own_s || own_0) {
-        for (int r = tid; r < NREG; r += Lay::NT) {
-            const int i = c.i0 - 1 + r % (TX + 2), j = c.j0 - 1 + r / (TX + 2);
-            if (i > c.n0 + 2 || j > c.n1 + 2 || !c.own_x(i) || !c.own_y(j)) continue;
-            if (own_s) {
-                const long long I = c.gidx(i, j, s);
-                out.P[I] = c.P(s, i, j);
-                out.txx[I] = c.Txx(s, i, j);
-                out.tyy[I] = c.Tyy(s, i, j);
-                out.tzz[I] = c.Tzz(s, i, j);
-                out.txy[I] = c.Txy(s, i, j);
-                out.txz[I] = c.Txz(s, i, j);
-                out.tyz[I] = c.Tyz(s, i, j);
-            }
-            if (own_0) {
-                const long long I0 = c.gidx(i, j, 0);
-                out.P[I0] = c.P(s - 1, i, j);  // own_0: s == 1, ghost plane 0
-                out.tzz[I0] = c.Tzz(s - 1, i, j);
-            }
-        }
-    }
-    // the V update of the same step reads the fixed-up plane
-    __syncthreads();
+#undef FI_LOAD
 }
 
-// ---- ghost / image writes: per dim a fixed three-entry list (own, low, high) ----
+// ---- new stresses at (li, lj): values only, stored by the caller ----------------------
+enum { F_P = 1, F_XX = 2, F_YY = 4, F_ZZ = 8 };
+
 template <typename T>
-struct Img {
-    int pos[3];
-    bool ok[3];
-    bool dir[3];  // Dirichlet ghost 2c - v (else copy)
-    T c[3];
+struct Centre {
+    T P, xx, yy, zz;
 };
 
-template <typename T>
-__device__ __forceinline__ Img<T> img_own(int q) {
-    Img<T> d;
-    d.pos[0] = q; d.ok[0] = true; d.dir[0] = false; d.c[0] = T(0);
-    d.pos[1] = 0; d.ok[1] = false; d.dir[1] = false; d.c[1] = T(0);
-    d.pos[2] = 0; d.ok[2] = false; d.dir[2] = false; d.c[2] = T(0);
-    return d;
+// P and the components of `mask` at plane s
+template <int mask, typename T, int TX, int TY>
+__device__ __forceinline__ Centre<T> centre_raw(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, int s, int li,
+                                                int lj, const Ptrs<T> &out) {
+    constexpr int BV = FBox<T, TX, TY, M_VX>::bw;
+    const T *vx = EL(M_VX, c.V0), *vy = EL(M_VY, c.V0), *vz = EL(M_VZ, c.V0), *vzp = EL(M_VZ, c.V1);
+    const T etac = *EL(M_ET, c.V0);
+    Centre<T> r;
+    const T oP = *EL(M_P, c.C);
+    T oXX = T(0), oYY = T(0), oZZ = T(0);
+    if (mask & F_XX) oXX = *EL(M_XX, c.C);
+    if (mask & F_YY) oYY = *EL(M_YY, c.C);
+    if (mask & F_ZZ) oZZ = *EL(M_ZZ, c.C);
+    const T exx = (vx[1] - vx[0]) * q.inv_dx[0];
+    const T eyy = (vy[BV] - vy[0]) * q.inv_dx[1];
+    const T ezz = (vzp[0] - vz[0]) * q.inv_dx[2];
+    const T divV = exx + eyy + ezz;
+    r.P = oP - (p.p_forcing ? divV + __ldg(out.fP + c.sxy * s + c.col(li, lj)) : divV) * etac * q.dt_P;
+    r.xx = oXX - (oXX - T(2.0) * etac * (exx - third(divV))) * q.dt_tau[0];
+    r.yy = oYY - (oYY - T(2.0) * etac * (eyy - third(divV))) * q.dt_tau[1];
+    r.zz = oZZ - (oZZ - T(2.0) * etac * (ezz - third(divV))) * q.dt_tau[2];
+    return r;
 }
-// Center-located value at index q (1..N) along a dim with BC kinds kl/kr; lo / hi:
-// the low / high ghost comes from elsewhere (a periodic image of this model's own
-// value, which a subdomain's halo exchange replaces with its neighbour's).
-// neumann: copies (η_next); else Velocity-BC ghosts 2c - v of a velocity component
+
+// τxy at plane s
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T xy_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj) {
+    constexpr int BV = FBox<T, TX, TY, M_VX>::bw;
+    const T *vx = EL(M_VX, c.V0), *vy = EL(M_VY, c.V0), *et = EL(M_ET, c.V0);
+    const T o = *EL(M_XY, c.C);
+    const T exy = T(0.5) * ((vy[0] - vy[-1]) * q.inv_dx[0] + (vx[0] - vx[-BV]) * q.inv_dx[1]);
+    const T e_xy = h(h(et[-1 - BV] + et[-BV]) + h(et[-1] + et[0]));
+    return o - (o - T(2.0) * e_xy * exy) * q.dt_tau[3];
+}
+
+// τxz and τyz at plane s + 1
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T xz_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj) {
+    const T *vx = EL(M_VX, c.V1), *vxm = EL(M_VX, c.V0), *vz = EL(M_VZ, c.V1);
+    const T *et = EL(M_ET, c.V1), *etm = EL(M_ET, c.V0);
+    const T o = *EL(M_XZ, c.V1);
+    const T exz = T(0.5) * ((vz[0] - vz[-1]) * q.inv_dx[0] + (vx[0] - vxm[0]) * q.inv_dx[2]);
+    const T e_xz = h(h(etm[-1] + etm[0]) + h(et[-1] + et[0]));
+    return o - (o - T(2.0) * e_xz * exz) * q.dt_tau[4];
+}
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T yz_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj) {
+    constexpr int BV = FBox<T, TX, TY, M_VX>::bw;
+    const T *vy = EL(M_VY, c.V1), *vym = EL(M_VY, c.V0), *vz = EL(M_VZ, c.V1);
+    const T *et = EL(M_ET, c.V1), *etm = EL(M_ET, c.V0);
+    const T o = *EL(M_YZ, c.V1);
+    const T eyz = T(0.5) * ((vz[0] - vz[-BV]) * q.inv_dx[1] + (vy[0] - vym[0]) * q.inv_dx[2]);
+    const T e_yz = h(h(etm[-BV] + etm[0]) + h(et[-BV] + et[0]));
+    return o - (o - T(2.0) * e_yz * eyz) * q.dt_tau[5];
+}
+
+// ---- boundary values of the shear stresses ------------------------------------------
+__device__ __forceinline__ bool stress_fixed(int kind) { return kind == FI_BC_TRACTION || kind == FI_BC_SLIP; }
+
+// fixed-node bits of a position
+template <typename T, int TX, int TY>
+__device__ __forceinline__ unsigned shear_flags(const Ctx<T, TX, TY> &c, const KParams &p, int i, int j) {
+    unsigned f = 0;
+    if (i == 1 && stress_fixed(p.bc_kind[0][0])) f |= CF_X0;
+    if (i == c.n0 + 1 && stress_fixed(p.bc_kind[0][1])) f |= CF_X1;
+    if (j == 1 && stress_fixed(p.bc_kind[1][0])) f |= CF_Y0;
+    if (j == c.n1 + 1 && stress_fixed(p.bc_kind[1][1])) f |= CF_Y1;
+    return f;
+}
+// x faces, then y faces, then z faces (a later dimension's value wins)
+template <typename T>
+__device__ __forceinline__ T fix_xy(const TConst<T> &q, T v, unsigned f) {
+    if (f & CF_X0) v = q.bc_val[0][0][1];
+    if (f & CF_X1) v = q.bc_val[0][1][1];
+    if (f & CF_Y0) v = q.bc_val[1][0][0];
+    if (f & CF_Y1) v = q.bc_val[1][1][0];
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T fix_xz(const TConst<T> &q, T v, unsigned f) {
+    if (f & CF_X0) v = q.bc_val[0][0][2];
+    if (f & CF_X1) v = q.bc_val[0][1][2];
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T fix_yz(const TConst<T> &q, T v, unsigned f) {
+    if (f & CF_Y0) v = q.bc_val[1][0][2];
+    if (f & CF_Y1) v = q.bc_val[1][1][2];
+    return v;
+}
+// the side of plane k's z face with fixed shear stresses, or -1
+template <typename T, int TX, int TY>
+__device__ __forceinline__ int z_fixed(const Ctx<T, TX, TY> &c, const KParams &p, int k) {
+    if (k == 1 && stress_fixed(p.bc_kind[2][0])) return 0;
+    if (k == c.n2 + 1 && stress_fixed(p.bc_kind[2][1])) return 1;
+    return -1;
+}
+
+// The ghosts of P and τxx (τyy) beside a traction side, from the values at the cell next
+// to it; written by the thread that computed those, where the ghost lies in this CTA's
+// column (or is its low ring).
+template <typename T, int TX, int TY>
+__device__ __forceinline__ void traction_x(const Ctx<T, TX, TY> &c, const TConst<T> &q, const Ptrs<T> &out, int s, int side,
+                                           int lj, T P, T xx, bool write) {
+    const int li = side == 0 ? -1 : c.n0 + 1 - c.i0;
+    const T tv = T(2.0) * q.bc_val[0][side][0];
+    *EL(M_P, c.C) = tv - P;
+    *EL(M_XX, c.C) = tv - xx;
+    if (write) {
+        const long long I = c.sxy * s + c.col(li, lj);
+        out.P[I] = tv - P;
+        out.txx[I] = tv - xx;
+    }
+}
+template <typename T, int TX, int TY>
+__device__ __forceinline__ void traction_y(const Ctx<T, TX, TY> &c, const TConst<T> &q, const Ptrs<T> &out, int s, int side,
+                                           int li, T P, T yy, bool write) {
+    const int lj = side == 0 ? -1 : c.n1 + 1 - c.j0;
+    const T tv = T(2.0) * q.bc_val[1][side][1];
+    *EL(M_P, c.C) = tv - P;
+    *EL(M_YY, c.C) = tv - yy;
+    if (write) {
+        const long long I = c.sxy * s + c.col(li, lj);
+        out.P[I] = tv - P;
+        out.tyy[I] = tv - yy;
+    }
+}
+
+// Ring stresses of step s, one side per warp on the last warps (one per scheduler for
+// 32-wide tiles): the row below (P, τyy), the row above (τxy, τyz), the column left
+// (P, τxx), the column right (τxy, τxz) with the corner above it (τxy).
+template <bool BND, typename T, int TX, int TY>
+__device__ __forceinline__ void sigma_ring(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &out,
+                                           int s, int zf, bool write) {
+    constexpr int RW = TX / 32, NW = Layout<T, TX, TY>::NW;
+    static_assert(TY < 32 && NW >= 2 * RW + 2, "one ring side per warp");
+    const int w = (int)(threadIdx.x / 32) - (NW - 2 * RW - 2), lane = threadIdx.x % 32;
+    const bool cz = s >= 1;  // s <= n2 in every step with stresses
+    if (w < 0) return;
+    if (w < RW) {
+        const int li = lane + 32 * w, lj = -1, i = c.i0 + li, j = c.j0 - 1;
+        if (cz && (!BND || ((i <= c.n0 || (c.hx1 && i == c.n0 + 1)) && (j >= 1 || c.hy0)))) {
+            const Centre<T> v = centre_raw<F_P | F_YY>(c, p, q, s, li, lj, out);
+            *EL(M_P, c.C) = v.P;
+            *EL(M_YY, c.C) = v.yy;
+            if (BND && j == 0 && write) {
+                const long long I = c.sxy * s + c.col(li, lj);
+                out.P[I] = v.P;
+                out.tyy[I] = v.yy;
+            }
+            if (BND && j == c.n1 && p.bc_kind[1][1] == FI_BC_TRACTION) traction_y(c, q, out, s, 1, li, v.P, v.yy, write);
+        }
+    } else if (w < 2 * RW) {
+        const int li = lane + 32 * (w - RW), lj = TY, i = c.i0 + li, j = c.j0 + TY;
+        if (!BND || (i <= c.n0 + 1 && j <= c.n1 + 1)) {
+            T xy = xy_raw(c, q, li, lj), yz = yz_raw(c, q, li, lj);
+            if (BND) {
+                const unsigned f = shear_flags(c, p, i, j);
+                xy = fix_xy(q, xy, f);
+                yz = fix_yz(q, yz, f);
+            }
+            if (zf >= 0) yz = q.bc_val[2][zf][1];
+            *EL(M_XY, c.C) = xy;
+            *EL(M_YZ, c.V1) = yz;
+        }
+    } else if (w == 2 * RW) {
+        const int li = -1, lj = lane, i = c.i0 - 1, j = c.j0 + lane;
+        if (lane < TY && cz && (!BND || ((i >= 1 || c.hx0) && (j <= c.n1 || (c.hy1 && j == c.n1 + 1))))) {
+            const Centre<T> v = centre_raw<F_P | F_XX>(c, p, q, s, li, lj, out);
+            *EL(M_P, c.C) = v.P;
+            *EL(M_XX, c.C) = v.xx;
+            if (BND && i == 0 && write) {
+                const long long I = c.sxy * s + c.col(li, lj);
+                out.P[I] = v.P;
+                out.txx[I] = v.xx;
+            }
+            if (BND && i == c.n0 && p.bc_kind[0][1] == FI_BC_TRACTION) traction_x(c, q, out, s, 1, lj, v.P, v.xx, write);
+        }
+    } else {
+        const int li = TX, lj = lane, i = c.i0 + TX, j = c.j0 + lane;
+        if (lane <= TY && (!BND || (i <= c.n0 + 1 && j <= c.n1 + 1))) {
+            T xy = xy_raw(c, q, li, lj), xz = T(0);
+            if (lane < TY) xz = xz_raw(c, q, li, lj);
+            if (BND) {
+                const unsigned f = shear_flags(c, p, i, j);
+                xy = fix_xy(q, xy, f);
+                xz = fix_xz(q, xz, f);
+            }
+            if (zf >= 0) xz = q.bc_val[2][zf][0];
+            *EL(M_XY, c.C) = xy;
+            if (lane < TY) *EL(M_XZ, c.V1) = xz;
+        }
+    }
+}
+
+// values of the thread's column that V.z needs from plane to plane
+template <typename T>
+struct Carry {
+    T P, zz;    // new values of the step's plane
+    T Pm, zzm;  // of the plane below
+    T etm;      // η of the plane below
+};
+
+// New stresses of step s at the thread's position.  wc: the centre stresses and τxy of
+// plane s belong to this z-block; wf: τxz, τyz of plane s + 1 do.
+template <bool BND, typename T, int TX, int TY>
+__device__ __forceinline__ void sigma_column(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &out,
+                                             int s, int li, int lj, unsigned fl, int zf, bool wc, bool wf, long long I,
+                                             Carry<T> &k) {
+    const bool cz = s >= 1;
+    const bool cx = !BND || (fl & CF_CX), cy = !BND || (fl & CF_CY);
+    const Centre<T> v = centre_raw<F_P | F_XX | F_YY | F_ZZ>(c, p, q, s, li, lj, out);
+    T xy = xy_raw(c, q, li, lj);
+    T xz = xz_raw(c, q, li, lj);
+    T yz = yz_raw(c, q, li, lj);
+    if (BND && (fl & CF_SHEAR)) {
+        xy = fix_xy(q, xy, fl);
+        xz = fix_xz(q, xz, fl);
+        yz = fix_yz(q, yz, fl);
+    }
+    if (zf >= 0) {
+        xz = q.bc_val[2][zf][0];
+        yz = q.bc_val[2][zf][1];
+    }
+    const bool dc = cx && cy && cz;
+    if (dc) {
+        *EL(M_P, c.C) = v.P;
+        *EL(M_XX, c.C) = v.xx;
+        *EL(M_YY, c.C) = v.yy;
+    }
+    *EL(M_XY, c.C) = xy;
+    *EL(M_XZ, c.V1) = xz;
+    *EL(M_YZ, c.V1) = yz;
+    k.P = v.P;
+    k.zz = v.zz;
+    if (wc) {
+        if (dc) {
+            out.P[I] = v.P;
+            out.txx[I] = v.xx;
+            out.tyy[I] = v.yy;
+            out.tzz[I] = v.zz;
+        }
+        if (!BND || (fl & CF_IN)) out.txy[I] = xy;
+    }
+    if (wf && (!BND || (fl & CF_IN))) {
+        if (cy) out.txz[I + c.sxy] = xz;
+        if (cx) out.tyz[I + c.sxy] = yz;
+    }
+    if (BND && dc && (fl & CF_TRAC)) {
+        if (fl & CF_TX0) traction_x(c, q, out, s, 0, lj, v.P, v.xx, wc);
+        if (fl & CF_TX1) traction_x(c, q, out, s, 1, lj, v.P, v.xx, wc);
+        if (fl & CF_TY0) traction_y(c, q, out, s, 0, li, v.P, v.yy, wc);
+        if (fl & CF_TY1) traction_y(c, q, out, s, 1, li, v.P, v.yy, wc);
+    }
+    // the ghosts under a traction bottom
+    if (s == 1 && p.bc_kind[2][0] == FI_BC_TRACTION) {
+        const T tv = T(2.0) * q.bc_val[2][0][2];
+        k.Pm = tv - v.P;
+        k.zzm = tv - v.zz;
+        if (wc && dc) {
+            out.P[I - c.sxy] = k.Pm;
+            out.tzz[I - c.sxy] = k.zzm;
+        }
+    }
+}
+
+// ---- ghost / image writes ---------------------------------------------------------------
+template <typename T>
+struct Img {
+    int d;     // offset along the dimension of the value's image beside it (0: none)
+    int d2;    // of a second one, a copy: next to one physical and one foreign side
+    bool dir;  // the first is a Dirichlet ghost 2c - v (else a copy)
+    T c;
+};
+
+// Center-located value at index q (1..N) along a dim with BC kinds kl/kr; lo / hi: the
+// low / high ghost comes from elsewhere (a periodic image of this model's own value,
+// which a subdomain's halo exchange replaces with its neighbour's).  neumann: copies
+// (η_next); else Velocity-BC ghosts 2c - v of a velocity component.  Dimensions have 3
+// or more cells.
 template <typename T>
 __device__ __forceinline__ Img<T> img_center(int q, int N, bool lo, bool hi, int kl, int kr, T cl, T cr, bool neumann) {
-    Img<T> d = img_own<T>(q);
-    if (lo) {
-        if (q == N) { d.pos[1] = 0; d.ok[1] = true; }
-    } else if (neumann) {
-        if (q == 1) { d.pos[1] = 0; d.ok[1] = true; }
-    } else if (q == 1 && kl == FI_BC_VELOCITY) {
-        d.pos[1] = 0; d.ok[1] = true; d.dir[1] = true; d.c[1] = cl;
-    }
-    if (hi) {
-        if (q == 1) { d.pos[2] = N + 1; d.ok[2] = true; }
-    } else if (neumann) {
-        if (q == N) { d.pos[2] = N + 1; d.ok[2] = true; }
-    } else if (q == N && kr == FI_BC_VELOCITY) {
-        d.pos[2] = N + 1; d.ok[2] = true; d.dir[2] = true; d.c[2] = cr;
-    }
-    return d;
+    Img<T> r{0, 0, false, T(0)};
+    if (q == 1 && !lo && (neumann || kl == FI_BC_VELOCITY)) r = {-1, 0, !neumann, cl};
+    if (q == N && !hi && (neumann || kr == FI_BC_VELOCITY)) r = {1, 0, !neumann, cr};
+    const int away = (q == N && lo) ? -N : (q == 1 && hi) ? N : 0;
+    (r.d ? r.d2 : r.d) = away;
+    return r;
 }
 template <typename T>
 __device__ __forceinline__ Img<T> img_vertex(int q, int N, bool lo, bool hi) {
-    Img<T> d = img_own<T>(q);
-    if (lo && q == N) { d.pos[1] = 0; d.ok[1] = true; }
-    if (hi && q == 1) { d.pos[2] = N + 1; d.ok[2] = true; }
-    if (hi && q == 2) { d.pos[2] = N + 2; d.ok[2] = true; }
-    return d;
+    Img<T> r{0, 0, false, T(0)};
+    if (lo && q == N) r.d = -N;
+    if (hi && (q == 1 || q == 2)) r.d = N;
+    return r;
 }
 
-template <typename T, typename C>
-__device__ __forceinline__ void write_images(const C &c, T *f, T v, const Img<T> &ix, const Img<T> &iy,
-                                             const Img<T> &iz) {
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        if (!ix.ok[a]) continue;
-        T va = ix.dir[a] ? T(2.0) * ix.c[a] - v : v;
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-            if (!iy.ok[b]) continue;
-            T vb = iy.dir[b] ? T(2.0) * iy.c[b] - va : va;
-#pragma unroll
-            for (int e = 0; e < 3; e++) {
-                if (!iz.ok[e]) continue;
-                T ve = iz.dir[e] ? T(2.0) * iz.c[e] - vb : vb;
-                f[c.gidx(ix.pos[a], iy.pos[b], iz.pos[e])] = ve;
-            }
+// the images of v (x, then y, then z: an image of an image follows both rules)
+template <typename T>
+__device__ __forceinline__ T img_value(const Img<T> &m, T v) { return m.dir ? T(2.0) * m.c - v : v; }
+
+template <typename T>
+__device__ __forceinline__ void put_images(T *f, T v, const Img<T> &x, const Img<T> &y, long long sx, const Img<T> &z,
+                                           long long sxy, bool dup) {
+    const T vx = img_value(x, v);
+    if (x.d) f[x.d] = vx;
+    if (y.d) {
+        T *fy = f + sx * y.d;
+        fy[0] = img_value(y, v);
+        if (x.d) fy[x.d] = img_value(y, vx);
+    }
+    if (z.d) {
+        T *fz = f + sxy * z.d;
+        fz[0] = img_value(z, v);
+        if (x.d) fz[x.d] = img_value(z, vx);
+        if (y.d) {
+            fz[sx * y.d] = img_value(z, img_value(y, v));
+            if (x.d) fz[sx * y.d + x.d] = img_value(z, img_value(y, vx));
         }
     }
-}
-
-// ---- velocity / η_next update of plane t on the column ----------------------------
-template <typename T, typename C>
-__device__ __forceinline__ T vx_raw(const C &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in, int t, int i,
-                                    int j, long long I) {
-    const T idx = q.inv_dx[0], idy = q.inv_dx[1], idz = q.inv_dx[2];
-    T gx = (p.g_kind[0] == FI_G_FIELD ? in.gx[I] : q.g_val[0]);
-    T ex = h(c.Eta(t, i - 1, j) + c.Eta(t, i, j));
-    return c.Vx(t, i, j) + div_fast(-(c.P(t, i, j) - c.P(t, i - 1, j)) * idx + (c.Txx(t, i, j) - c.Txx(t, i - 1, j)) * idx +
-                                       (c.Txy(t, i, j + 1) - c.Txy(t, i, j)) * idy +
-                                       (c.Txz(t + 1, i, j) - c.Txz(t, i, j)) * idz - gx,
-                                   ex) *
-                               q.dt_V[0];
-}
-template <typename T, typename C>
-__device__ __forceinline__ T vy_raw(const C &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in, int t, int i,
-                                    int j, long long I) {
-    const T idx = q.inv_dx[0], idy = q.inv_dx[1], idz = q.inv_dx[2];
-    T gy = (p.g_kind[1] == FI_G_FIELD ? in.gy[I] : q.g_val[1]);
-    T ey = h(c.Eta(t, i, j - 1) + c.Eta(t, i, j));
-    return c.Vy(t, i, j) + div_fast(-(c.P(t, i, j) - c.P(t, i, j - 1)) * idy + (c.Tyy(t, i, j) - c.Tyy(t, i, j - 1)) * idy +
-                                       (c.Txy(t, i + 1, j) - c.Txy(t, i, j)) * idx +
-                                       (c.Tyz(t + 1, i, j) - c.Tyz(t, i, j)) * idz - gy,
-                                   ey) *
-                               q.dt_V[1];
-}
-template <typename T, typename C>
-__device__ __forceinline__ T vz_raw(const C &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in, int t, int i,
-                                    int j, long long I) {
-    const T idx = q.inv_dx[0], idy = q.inv_dx[1], idz = q.inv_dx[2];
-    T gz = (p.g_kind[2] == FI_G_FIELD ? in.gz[I] : q.g_val[2]);
-    T ez = h(c.Eta(t - 1, i, j) + c.Eta(t, i, j));
-    return c.Vz(t, i, j) + div_fast(-(c.P(t, i, j) - c.P(t - 1, i, j)) * idz + (c.Tzz(t, i, j) - c.Tzz(t - 1, i, j)) * idz +
-                                       (c.Txz(t, i + 1, j) - c.Txz(t, i, j)) * idx +
-                                       (c.Tyz(t, i, j + 1) - c.Tyz(t, i, j)) * idy - gz,
-                                   ez) *
-                               q.dt_V[2];
-}
-template <typename T, typename C>
-__device__ __forceinline__ T eta_raw(const C &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in, int t, int i,
-                                     int j, long long I) {
-    T xx = c.Txx(t, i, j), yy = c.Tyy(t, i, j), zz = c.Tzz(t, i, j);
-    T lxy = h(h(c.Txy(t, i, j) + c.Txy(t, i + 1, j)) + h(c.Txy(t, i, j + 1) + c.Txy(t, i + 1, j + 1)));
-    T lxz = h(h(c.Txz(t, i, j) + c.Txz(t, i + 1, j)) + h(c.Txz(t + 1, i, j) + c.Txz(t + 1, i + 1, j)));
-    T lyz = h(h(c.Tyz(t, i, j) + c.Tyz(t, i, j + 1)) + h(c.Tyz(t + 1, i, j) + c.Tyz(t + 1, i, j + 1)));
-    T s2 = T(0.5) * (xx * xx + yy * yy + zz * zz) + lxy * lxy + lxz * lxz + lyz * lyz;
-    return rheology_s2(p, q.rheo_A, q.rheo_inv_eta_reg, in.eta_lin, in.A, c.Eta(t, i, j), I, s2);
-}
-
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void v_point(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q,
-                                        const Ptrs<T> &in, const Ptrs<T> &out, int t, int i, int j) {
-    const int n0 = c.n0, n1 = c.n1, n2 = c.n2;
-    if (i > n0 + 1 || j > n1 + 1) return;
-    const long long I = c.gidx(i, j, t);
-    const bool near = i <= 2 || i >= n0 || j <= 2 || j >= n1 || t <= 1 || t >= n2;
-    if (!near) {
-        // all four values before the first store (see sigma_point)
-        const T vxn = vx_raw(c, p, q, in, t, i, j, I);
-        const T vyn = vy_raw(c, p, q, in, t, i, j, I);
-        const T vzn = vz_raw(c, p, q, in, t, i, j, I);
-        const T etn = p.freeze_eta ? T(0) : eta_raw(c, p, q, in, t, i, j, I);
-        out.Vx[I] = vxn;
-        out.Vy[I] = vyn;
-        out.Vz[I] = vzn;
-        if (!p.freeze_eta) out.eta_next[I] = etn;
-        return;
+    if (!dup) return;
+    // second images (a physical and a foreign side): copies, with the first images of the
+    // other dimensions
+#pragma unroll 1
+    for (int e = 0; e < 18; e++) {
+        const int a = e % 3, b = (e / 3) % 3, g = e / 9;
+        const int da = a == 0 ? 0 : a == 1 ? x.d : x.d2, db = b == 0 ? 0 : b == 1 ? y.d : y.d2, dg = g ? z.d : 0;
+        if ((a != 2 && b != 2) || (a && !da) || (b && !db) || (g && !dg)) continue;
+        T u = a == 1 ? img_value(x, v) : v;
+        u = b == 1 ? img_value(y, u) : u;
+        u = g == 1 ? img_value(z, u) : u;
+        f[da + sx * db + sxy * dg] = u;
     }
-    auto node_fixed = [](int kind) { return kind == FI_BC_SLIP || kind == FI_BC_VELOCITY; };
+}
+
+// ---- velocity / η_next update of plane t on the column ----------------------------------
+// The thread's neighbours in shared memory; P, τzz and η of the plane below from Carry.
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T vx_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj, T gx) {
+    constexpr int BY = FBox<T, TX, TY, M_XY>::bw;
+    const T *P = EL(M_P, c.C), *xx = EL(M_XX, c.C), *xy = EL(M_XY, c.C), *et = EL(M_ET, c.V0);
+    const T ex = h(et[-1] + et[0]);
+    return *EL(M_VX, c.V0) +
+           div_fast(-(P[0] - P[-1]) * q.inv_dx[0] + (xx[0] - xx[-1]) * q.inv_dx[0] + (xy[BY] - xy[0]) * q.inv_dx[1] +
+                        (*EL(M_XZ, c.V1) - *EL(M_XZ, c.V0)) * q.inv_dx[2] - gx,
+                    ex) *
+               q.dt_V[0];
+}
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T vy_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj, T gy) {
+    constexpr int BP = FBox<T, TX, TY, M_P>::bw, BYY = FBox<T, TX, TY, M_YY>::bw, BV = FBox<T, TX, TY, M_ET>::bw;
+    const T *P = EL(M_P, c.C), *yy = EL(M_YY, c.C), *xy = EL(M_XY, c.C), *et = EL(M_ET, c.V0);
+    const T ey = h(et[-BV] + et[0]);
+    return *EL(M_VY, c.V0) +
+           div_fast(-(P[0] - P[-BP]) * q.inv_dx[1] + (yy[0] - yy[-BYY]) * q.inv_dx[1] + (xy[1] - xy[0]) * q.inv_dx[0] +
+                        (*EL(M_YZ, c.V1) - *EL(M_YZ, c.V0)) * q.inv_dx[2] - gy,
+                    ey) *
+               q.dt_V[1];
+}
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T vz_raw(const Ctx<T, TX, TY> &c, const TConst<T> &q, int li, int lj, T gz, const Carry<T> &k) {
+    constexpr int BYZ = FBox<T, TX, TY, M_YZ>::bw;
+    const T *xz = EL(M_XZ, c.V0), *yz = EL(M_YZ, c.V0);
+    const T ez = h(k.etm + *EL(M_ET, c.V0));
+    return *EL(M_VZ, c.V0) +
+           div_fast(-(k.P - k.Pm) * q.inv_dx[2] + (k.zz - k.zzm) * q.inv_dx[2] + (xz[1] - xz[0]) * q.inv_dx[0] +
+                        (yz[BYZ] - yz[0]) * q.inv_dx[1] - gz,
+                    ez) *
+               q.dt_V[2];
+}
+template <typename T, int TX, int TY>
+__device__ __forceinline__ T eta_raw(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in, int li,
+                                     int lj, long long I, T zz) {
+    // a linear viscosity without regularisation or relaxation does not read the stresses
+    if (linear_unrelaxed(p)) return p.rheo_eta_is_field ? in.eta_lin[I] : T(p.rheo_eta);
+    constexpr int BY = FBox<T, TX, TY, M_XY>::bw, BYZ = FBox<T, TX, TY, M_YZ>::bw;
+    const T xx = *EL(M_XX, c.C), yy = *EL(M_YY, c.C);
+    const T *xy = EL(M_XY, c.C);
+    const T *xz = EL(M_XZ, c.V0), *xzp = EL(M_XZ, c.V1), *yz = EL(M_YZ, c.V0), *yzp = EL(M_YZ, c.V1);
+    const T lxy = h(h(xy[0] + xy[1]) + h(xy[BY] + xy[BY + 1]));
+    const T lxz = h(h(xz[0] + xz[1]) + h(xzp[0] + xzp[1]));
+    const T lyz = h(h(yz[0] + yz[BYZ]) + h(yzp[0] + yzp[BYZ]));
+    const T s2 = T(0.5) * (xx * xx + yy * yy + zz * zz) + lxy * lxy + lxz * lxz + lyz * lyz;
+    return rheology_s2(p, q.rheo_A, q.rheo_inv_eta_reg, in.eta_lin, in.A, *EL(M_ET, c.V0), I, s2);
+}
+
+__device__ __forceinline__ bool node_fixed(int kind) { return kind == FI_BC_SLIP || kind == FI_BC_VELOCITY; }
+
+// the ghost images of the four values at (t, i, j)
+template <typename T, int TX, int TY>
+__device__ __forceinline__ void v_images(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &out,
+                                         int t, int li, int lj, unsigned fl, long long I, T vx, T vy, T vz, T et) {
+    const int n0 = c.n0, n1 = c.n1, n2 = c.n2, i = c.i0 + li, j = c.j0 + lj;
     const int xl = p.bc_kind[0][0], xr = p.bc_kind[0][1], yl = p.bc_kind[1][0], yr = p.bc_kind[1][1];
     const int zl = p.bc_kind[2][0], zr = p.bc_kind[2][1];
-    // ---- V.x at (V, C, C)
-    if (j <= n1 && t >= 1 && t <= n2 && !(c.hx1 && i == n0 + 1)) {
-        T v;
-        if (!c.hx0 && i == 1 && node_fixed(xl)) v = q.bc_val[0][0][0];
-        else if (!c.hx1 && i == n0 + 1 && node_fixed(xr)) v = q.bc_val[0][1][0];
-        else v = vx_raw(c, p, q, in, t, i, j, I);
-        write_images(c, out.Vx, v, img_vertex<T>(i, n0, c.hx0, c.hx1),
-                     img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, q.bc_val[1][0][0], q.bc_val[1][1][0], false),
-                     img_center<T>(t, n2, false, false, zl, zr, q.bc_val[2][0][0], q.bc_val[2][1][0], false));
-    }
+    const bool cz = t <= n2, dup = fl & CF_DUP;
+    const bool y_node = fl & (CF_VY0 | CF_VY1), z_node = (t == 1 && node_fixed(zl)) || (t == n2 + 1 && node_fixed(zr));
     // A value on a fixed node of its own dim d is written there last by the
     // reference's dim-d node assignment, which spans the ghosts of the dims before
     // d: its images along those dims are copies, not mirrors (as_copies).
-    auto as_copies = [](Img<T> d) {
-        d.dir[1] = false;
-        d.dir[2] = false;
-        return d;
+    auto as_copies = [](Img<T> m, bool yes) {
+        m.dir = m.dir && !yes;
+        return m;
     };
-    // ---- V.y at (C, V, C)
-    if (i <= n0 && t >= 1 && t <= n2 && !(c.hy1 && j == n1 + 1)) {
-        T v;
-        const bool y_node = (!c.hy0 && j == 1 && node_fixed(yl)) || (!c.hy1 && j == n1 + 1 && node_fixed(yr));
-        if (!c.hy0 && j == 1 && node_fixed(yl)) v = q.bc_val[1][0][1];
-        else if (!c.hy1 && j == n1 + 1 && node_fixed(yr)) v = q.bc_val[1][1][1];
-        else v = vy_raw(c, p, q, in, t, i, j, I);
-        Img<T> ix = img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, q.bc_val[0][0][1], q.bc_val[0][1][1], false);
-        write_images(c, out.Vy, v, y_node ? as_copies(ix) : ix, img_vertex<T>(j, n1, c.hy0, c.hy1),
-                     img_center<T>(t, n2, false, false, zl, zr, q.bc_val[2][0][1], q.bc_val[2][1][1], false));
-    }
-    // ---- V.z at (C, C, V)
-    if (i <= n0 && j <= n1 && t >= 1 && t <= n2 + 1) {
-        T v;
-        const bool z_node = (t == 1 && node_fixed(zl)) || (t == n2 + 1 && node_fixed(zr));
-        if (t == 1 && node_fixed(zl)) v = q.bc_val[2][0][2];
-        else if (t == n2 + 1 && node_fixed(zr)) v = q.bc_val[2][1][2];
-        else v = vz_raw(c, p, q, in, t, i, j, I);
-        Img<T> ix = img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, q.bc_val[0][0][2], q.bc_val[0][1][2], false);
-        Img<T> iy = img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, q.bc_val[1][0][2], q.bc_val[1][1][2], false);
-        write_images(c, out.Vz, v, z_node ? as_copies(ix) : ix, z_node ? as_copies(iy) : iy, img_own<T>(t));
-    }
-    // ---- η_next at (C, C, C), Neumann / periodic ghosts
-    if (!p.freeze_eta && i <= n0 && j <= n1 && t >= 1 && t <= n2) {
-        T en = eta_raw(c, p, q, in, t, i, j, I);
-        write_images(c, out.eta_next, en, img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, T(0), T(0), true),
-                     img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, T(0), T(0), true),
-                     img_center<T>(t, n2, false, false, zl, zr, T(0), T(0), true));
-    }
+    const Img<T> none{0, 0, false, T(0)};
+    if ((fl & CF_ONX) && cz)  // V.x at (V, C, C)
+        put_images(out.Vx + I, vx, img_vertex<T>(i, n0, c.hx0, c.hx1),
+                   img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, q.bc_val[1][0][0], q.bc_val[1][1][0], false), c.sx,
+                   img_center<T>(t, n2, false, false, zl, zr, q.bc_val[2][0][0], q.bc_val[2][1][0], false), c.sxy, dup);
+    if ((fl & CF_ONY) && cz)  // V.y at (C, V, C)
+        put_images(out.Vy + I, vy,
+                   as_copies(img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, q.bc_val[0][0][1], q.bc_val[0][1][1], false), y_node),
+                   img_vertex<T>(j, n1, c.hy0, c.hy1), c.sx,
+                   img_center<T>(t, n2, false, false, zl, zr, q.bc_val[2][0][1], q.bc_val[2][1][1], false), c.sxy, dup);
+    if (fl & CF_ONC)  // V.z at (C, C, V)
+        put_images(out.Vz + I, vz,
+                   as_copies(img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, q.bc_val[0][0][2], q.bc_val[0][1][2], false), z_node),
+                   as_copies(img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, q.bc_val[1][0][2], q.bc_val[1][1][2], false), z_node),
+                   c.sx, none, c.sxy, dup);
+    if (!p.freeze_eta && (fl & CF_ONC) && cz)  // η_next at (C, C, C), Neumann / periodic ghosts
+        put_images(out.eta_next + I, et, img_center<T>(i, n0, c.hx0, c.hx1, xl, xr, T(0), T(0), true),
+                   img_center<T>(j, n1, c.hy0, c.hy1, yl, yr, T(0), T(0), true), c.sx,
+                   img_center<T>(t, n2, false, false, zl, zr, T(0), T(0), true), c.sxy, dup);
 }
 
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void v_plane(const Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q,
-                                        const Ptrs<T> &in, const Ptrs<T> &out, int t) {
-    const int lane = threadIdx.x % 32, j = c.j0 + (int)(threadIdx.x / 32);
-#pragma unroll
-    for (int u = 0; u < TX / 32; u++) v_point(c, p, q, in, out, t, c.i0 + lane + 32 * u, j);
+// V and η_next of plane t.  Every value is computed (its operands lie in the boxes even
+// where no such point exists), then replaced at fixed nodes and stored where it exists.
+template <bool BND, typename T, int TX, int TY>
+__device__ __forceinline__ void v_column(const Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
+                                         const Ptrs<T> &out, int t, int li, int lj, unsigned fl, long long I, const Carry<T> &k,
+                                         T gx, T gy, T gz) {
+    const bool cz = t <= c.n2;
+    T vxn = vx_raw(c, q, li, lj, gx);
+    T vyn = vy_raw(c, q, li, lj, gy);
+    T vzn = vz_raw(c, q, li, lj, gz, k);
+    const bool on_c = !BND || (fl & CF_ONC);
+    T etn = T(0);
+    if (!p.freeze_eta && on_c && cz) etn = eta_raw(c, p, q, in, li, lj, I, k.zz);
+    if (BND) {
+        if (fl & CF_VX0) vxn = q.bc_val[0][0][0];
+        if (fl & CF_VX1) vxn = q.bc_val[0][1][0];
+        if (fl & CF_VY0) vyn = q.bc_val[1][0][1];
+        if (fl & CF_VY1) vyn = q.bc_val[1][1][1];
+    }
+    if (t == 1 && node_fixed(p.bc_kind[2][0])) vzn = q.bc_val[2][0][2];
+    if (!cz && node_fixed(p.bc_kind[2][1])) vzn = q.bc_val[2][1][2];
+    if (cz) {
+        if (!BND || (fl & CF_ONX)) out.Vx[I] = vxn;
+        if (!BND || (fl & CF_ONY)) out.Vy[I] = vyn;
+        if (!p.freeze_eta && on_c) out.eta_next[I] = etn;
+    }
+    if (on_c) out.Vz[I] = vzn;
+    if (t == 1 || t >= c.n2 || (BND && (fl & CF_IMG))) v_images(c, p, q, out, t, li, lj, fl, I, vxn, vyn, vzn, etn);
 }
 
-// the plane march of one CTA (TRIM: an interior column of a trimmed launch shape)
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void sweep(Ctx<T, TX, TY, TRIM> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
-                                      const Ptrs<T> &out, const InMaps &maps, uint64_t *bars, int *err) {
+// body force at a point of V; loaded ahead of the step's barrier
+template <typename T>
+__device__ __forceinline__ T body_force(const KParams &p, const TConst<T> &q, const T *g, int d, long long I) {
+    return p.g_kind[d] == FI_G_FIELD ? __ldg(g + I) : q.g_val[d];
+}
+
+template <typename T, int TX, int TY>
+__device__ __forceinline__ unsigned column_flags(const Ctx<T, TX, TY> &c, const KParams &p, int i, int j) {
+    if (i > c.n0 + 1 || j > c.n1 + 1) return 0u;
+    unsigned f = CF_IN | shear_flags(c, p, i, j);
+    const int xl = p.bc_kind[0][0], xr = p.bc_kind[0][1], yl = p.bc_kind[1][0], yr = p.bc_kind[1][1];
+    if (i <= c.n0 || c.hx1) f |= CF_CX;
+    if (j <= c.n1 || c.hy1) f |= CF_CY;
+    if (xl == FI_BC_TRACTION && i == 1) f |= CF_TX0;
+    if (xr == FI_BC_TRACTION && i == c.n0 && c.n0 + 1 < c.i0 + TX) f |= CF_TX1;
+    if (yl == FI_BC_TRACTION && j == 1) f |= CF_TY0;
+    if (yr == FI_BC_TRACTION && j == c.n1 && c.n1 + 1 < c.j0 + TY) f |= CF_TY1;
+    if (!c.hx0 && i == 1 && node_fixed(xl)) f |= CF_VX0;
+    if (!c.hx1 && i == c.n0 + 1 && node_fixed(xr)) f |= CF_VX1;
+    if (!c.hy0 && j == 1 && node_fixed(yl)) f |= CF_VY0;
+    if (!c.hy1 && j == c.n1 + 1 && node_fixed(yr)) f |= CF_VY1;
+    if (j <= c.n1 && !(c.hx1 && i == c.n0 + 1)) f |= CF_ONX;
+    if (i <= c.n0 && !(c.hy1 && j == c.n1 + 1)) f |= CF_ONY;
+    if (i <= c.n0 && j <= c.n1) f |= CF_ONC;
+    if (i <= 2 || i >= c.n0 || j <= 2 || j >= c.n1) f |= CF_IMG;
+    if (c.hx0 != c.hx1 || c.hy0 != c.hy1) f |= CF_DUP;
+    return f;
+}
+
+// the plane march of one CTA (BND: the column touches an x or y boundary)
+template <bool BND, typename T, int TX, int TY>
+__device__ __forceinline__ void sweep(Ctx<T, TX, TY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
+                                      const Ptrs<T> &out, const InMaps &maps, uint64_t *bars, unsigned *released, int *err) {
+    constexpr int NW = Layout<T, TX, TY>::NW;
     const int tid = threadIdx.x;
-    const int f = max(c.kb - 1, 1), last = min(c.ke, c.n2 + 1);
-    uint32_t phase = 0;  // bit b: parity of the next completion of bars[b]
-    c.set_plane(f);
+    const int li = tid % TX, lj = tid / TX;
+    const int first = c.kb - 1;
+    const int last = min(c.ke - 1, c.n2);  // last step that computes stresses
+    const int gmax = last + 1;             // last group it needs
     if (tid == 0) {
-        issue_group(c, maps, f - 1, false, &bars[(f - 1) % kBars]);
-        issue_group(c, maps, f, true, &bars[f % kBars]);
+        issue_group(c, maps, first, 0, bars);
+        issue_group(c, maps, first + 1, 1, bars);
+        if (first + 2 <= gmax) issue_group(c, maps, first + 2, 2, bars);
     }
-    auto wait_group = [&](int pl) -> bool {
-        const int b = pl % kBars;
-        bool ok = mbar_wait(&bars[b], (phase >> b) & 1u);
+    const unsigned fl = BND ? column_flags(c, p, c.i0 + li, c.j0 + lj) : (CF_ONX | CF_ONY | CF_ONC);
+    const bool inside = !BND || (fl & CF_IN);
+    uint32_t phase = 0;  // bit b: parity of the next completion of bars[b]
+    auto wait_group = [&](int g) -> bool {
+        const int b = g % 3;
+        const bool ok = mbar_wait(&bars[b], (phase >> b) & 1u);
         phase ^= 1u << b;
         return ok;
     };
-    bool ok = wait_group(f - 1);
-    for (int s = f; s <= last && ok; s++) {
+    Carry<T> k{T(0), T(0), T(0), T(0), T(0)};
+    long long I = c.sxy * first + c.col(li, lj);
+    bool ok = wait_group(first);
+    for (int s = first; s <= last && ok; s++, I += c.sxy) {
         c.set_plane(s);
-        if (tid == 0 && s + 1 <= last) {
-            fence_proxy_async();
-            issue_group(c, maps, s + 1, true, &bars[(s + 1) % kBars]);
-        }
-        ok = wait_group(s);
+        const bool own = s >= c.kb;
+        const int zf = z_fixed(c, p, s + 1);
+        ok = wait_group(s + 1);
         if (!ok) break;
-        sigma_plane(c, p, q, out, s);
-        if (s - 1 >= c.kb && s - 1 < c.ke) v_plane(c, p, q, in, out, s - 1);
-        __syncthreads();
+        sigma_column<BND>(c, p, q, out, s, li, lj, fl, zf, own, s + 1 < c.ke, I, k);
+        sigma_ring<BND>(c, p, q, out, s, zf, own);
+        if (own) {
+            T gx = q.g_val[0], gy = q.g_val[1], gz = q.g_val[2];
+            if (inside) {
+                gx = body_force(p, q, in.gx, 0, I);
+                gy = body_force(p, q, in.gy, 1, I);
+                gz = body_force(p, q, in.gz, 2, I);
+            }
+            __syncthreads();
+            v_column<BND>(c, p, q, in, out, s, li, lj, fl, I, k, gx, gy, gz);
+        }
+        k.Pm = k.P;
+        k.zzm = k.zz;
+        k.etm = *EL(M_ET, c.V0);
+        // the warp is done with the slots of this step; the last one to say so refills them
+        __syncwarp();
+        if (s + 3 <= gmax && tid % 32 == 0) {
+            unsigned n;
+            asm volatile("atom.add.acq_rel.cta.shared::cta.u32 %0, [%1], 1;" : "=r"(n) : "r"(smem_u32(released)) : "memory");
+            if (n % NW == NW - 1) {
+                fence_proxy_async();
+                issue_group(c, maps, s + 3, 2, bars);
+            }
+        }
     }
     if (ok) {
-        if (c.ke - 1 == last && last == c.n2 + 1) {
-            c.set_plane(last);
-            v_plane(c, p, q, in, out, last);
+        if (c.ke - 1 == c.n2 + 1) {
+            // the top plane of vertices: V.z, and the ghosts over a traction top
+            const int t = c.n2 + 1;
+            c.set_plane(t);
+            if (c.kb == t) __syncthreads();  // no step before this one had a barrier
+            if (inside && p.bc_kind[2][1] == FI_BC_TRACTION) {
+                const T tv = T(2.0) * q.bc_val[2][1][2];
+                k.P = tv - k.Pm;
+                k.zz = tv - k.zzm;
+                if (!BND || ((fl & CF_CX) && (fl & CF_CY))) {
+                    out.P[I] = k.P;
+                    out.tzz[I] = k.zz;
+                }
+            }
+            const T gz = inside ? body_force(p, q, in.gz, 2, I) : T(0);
+            v_column<BND>(c, p, q, in, out, t, li, lj, fl, I, k, T(0), T(0), gz);
         }
         return;
     }
@@ -762,6 +817,7 @@ __device__ __forceinline__ void sweep(Ctx<T, TX, TY, TRIM> &c, const KParams &p,
     atomicExch(err, (int)FI_ERR_TIMEOUT);
     for (int b = 0; b < kBars; b++) mbar_wait(&bars[b], (phase >> b) & 1u);
 }
+#undef EL
 
 // Tiles of one launch along a split dimension: a launch runs either every tile, or
 // part of them (the overlapped halo exchange runs the tiles next to the split faces
@@ -781,9 +837,9 @@ __device__ __forceinline__ int tile_y(const TileMap &tm) {
     return tm.dim == 1 ? b + tm.base + (b >= tm.nlow ? tm.shift : 0) : b;
 }
 
-template <typename T, int TX, int TY, bool TRIM>
-__device__ __forceinline__ void init_ctx(Ctx<T, TX, TY, TRIM> &c, const Geom &g, const KParams &p, unsigned char *smem,
-                                         int zb, const TileMap &tm) {
+template <typename T, int TX, int TY>
+__device__ __forceinline__ void init_ctx(Ctx<T, TX, TY> &c, const Geom &g, const KParams &p, unsigned char *smem, int zb,
+                                         const TileMap &tm) {
     c.sm = reinterpret_cast<T *>(smem);
     c.i0 = 1 + tile_x(tm) * TX;
     c.j0 = 1 + tile_y(tm) * TY;
@@ -799,13 +855,9 @@ __device__ __forceinline__ void init_ctx(Ctx<T, TX, TY, TRIM> &c, const Geom &g,
     c.hx1 = away(p.bc_kind[0][1]);
     c.hy0 = away(p.bc_kind[1][0]);
     c.hy1 = away(p.bc_kind[1][1]);
-    c.bnd_x = c.i0 == 1 || c.i0 + TX >= c.n0 + 1;
-    c.bnd_y = c.j0 == 1 || c.j0 + TY >= c.n1 + 1;
 }
 
-// TRIMK: the kernel holds the trimmed path for interior columns (shapes without it keep
-// one plane-march body, as small as before trimming existed)
-template <typename T, int TX, int TY, bool TRIMK>
+template <typename T, int TX, int TY>
 __global__ void __launch_bounds__(Layout<T, TX, TY>::NT, Layout<T, TX, TY>::MINB)
     fused3d_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, const __grid_constant__ InMaps maps, int zb,
                    TileMap tm, int *err) {
@@ -813,23 +865,19 @@ __global__ void __launch_bounds__(Layout<T, TX, TY>::NT, Layout<T, TX, TY>::MINB
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // the grid is padded to whole clusters: columns past the vertex range have no work
     if (1 + tile_x(tm) * TX > g.n[0] + 1 || 1 + tile_y(tm) * TY > g.n[1] + 1) return;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (size_t)S_COUNT * Lay::SLOT * sizeof(T));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (size_t)Lay::ELEMS * sizeof(T));
+    unsigned *released = reinterpret_cast<unsigned *>(bars + kBars);
     if (threadIdx.x == 0) {
         for (int b = 0; b < kBars; b++) mbar_init(&bars[b], 1);
+        *released = 0u;
         mbar_fence_init();
     }
     __syncthreads();
-    Ctx<T, TX, TY, false> c;
+    Ctx<T, TX, TY> c;
     init_ctx(c, g, p, smem_raw, zb, tm);
-    if constexpr (TRIMK) {
-        if (!c.bnd_x && !c.bnd_y) {
-            Ctx<T, TX, TY, true> ct;
-            init_ctx(ct, g, p, smem_raw, zb, tm);
-            sweep(ct, p, q, in, out, maps, bars, err);
-            return;
-        }
-    }
-    sweep(c, p, q, in, out, maps, bars, err);
+    // interior columns: no range tests, no x or y boundary values, no images
+    if (c.i0 > 2 && c.i0 + TX <= c.n0 && c.j0 > 2 && c.j0 + TY <= c.n1) sweep<false>(c, p, q, in, out, maps, bars, released, err);
+    else sweep<true>(c, p, q, in, out, maps, bars, released, err);
 }
 
 template <typename T, int TX, int TY>
@@ -838,12 +886,12 @@ cudaError_t launch_variant(const Geom &g, const KParams &p, const Ptrs<T> &in, c
     using Lay = Layout<T, TX, TY>;
     int dev = 0;
     cudaGetDevice(&dev);
-    static bool attr_set[2][64] = {};
-    if (dev < 64 && !attr_set[v.trim][dev]) {
-        cudaError_t e = cudaFuncSetAttribute(v.trim ? fused3d_kernel<T, TX, TY, true> : fused3d_kernel<T, TX, TY, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::SMEM);
+    static bool attr_set[64] = {};
+    if (dev < 64 && !attr_set[dev]) {
+        cudaError_t e =
+            cudaFuncSetAttribute(fused3d_kernel<T, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::SMEM);
         if (e != cudaSuccess) return e;
-        attr_set[v.trim][dev] = true;
+        attr_set[dev] = true;
     }
     auto up = [](int a, int b) { return (a + b - 1) / b * b; };
     TileMap tm{-1, 0, 1 << 30, 0};
@@ -884,13 +932,12 @@ cudaError_t launch_variant(const Geom &g, const KParams &p, const Ptrs<T> &in, c
         cfg.numAttrs = 1;
     }
     const TConst<T> q = make_tconst<T>(p);
-    if (v.trim) return cudaLaunchKernelEx(&cfg, fused3d_kernel<T, TX, TY, true>, g, p, q, in, out, maps, v.zb, tm, err);
-    return cudaLaunchKernelEx(&cfg, fused3d_kernel<T, TX, TY, false>, g, p, q, in, out, maps, v.zb, tm, err);
+    return cudaLaunchKernelEx(&cfg, fused3d_kernel<T, TX, TY>, g, p, q, in, out, maps, v.zb, tm, err);
 }
 
 template <typename T>
 size_t variant_smem(const Variant &v) {
-    if (v.tx == 64) return v.ty == 4 ? Layout<T, 64, 4>::SMEM : Layout<T, 64, 8>::SMEM;
+    if (v.tx == 64) return Layout<T, 64, 8>::SMEM;
     return v.ty == 4 ? Layout<T, 32, 4>::SMEM : v.ty == 16 ? Layout<T, 32, 16>::SMEM : Layout<T, 32, 8>::SMEM;
 }
 
@@ -906,18 +953,13 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encoder() {
     return fn;
 }
 
-// box (width, height) of input field f for tile tx x ty (trimmed: the interior box)
+// box (width, height) of input field f for tile tx x ty
 template <typename T, int TX, int TY>
-void box_of(int f, bool trimmed, int *bw, int *bh) {
-#define FI_BOX_CASE(F)                                      \
-    case F:                                                 \
-        if (trimmed) {                                      \
-            *bw = FBox<T, TX, TY, true, F>::bw;             \
-            *bh = FBox<T, TX, TY, true, F>::bh;             \
-        } else {                                            \
-            *bw = FBox<T, TX, TY, false, F>::bw;            \
-            *bh = FBox<T, TX, TY, false, F>::bh;            \
-        }                                                   \
+void box_of(int f, int *bw, int *bh) {
+#define FI_BOX_CASE(F)                 \
+    case F:                            \
+        *bw = FBox<T, TX, TY, F>::bw;  \
+        *bh = FBox<T, TX, TY, F>::bh;  \
         return;
     switch (f) {
         FI_BOX_CASE(M_P)
@@ -933,17 +975,11 @@ void box_of(int f, bool trimmed, int *bw, int *bh) {
 }
 
 template <typename T>
-void variant_box(const Variant &v, int f, bool trimmed, int *bw, int *bh) {
-    if (v.tx == 64) {
-        if (v.ty == 4) box_of<T, 64, 4>(f, trimmed, bw, bh);
-        else box_of<T, 64, 8>(f, trimmed, bw, bh);
-    } else if (v.ty == 4) {
-        box_of<T, 32, 4>(f, trimmed, bw, bh);
-    } else if (v.ty == 16) {
-        box_of<T, 32, 16>(f, trimmed, bw, bh);
-    } else {
-        box_of<T, 32, 8>(f, trimmed, bw, bh);
-    }
+void variant_box(const Variant &v, int f, int *bw, int *bh) {
+    if (v.tx == 64) box_of<T, 64, 8>(f, bw, bh);
+    else if (v.ty == 4) box_of<T, 32, 4>(f, bw, bh);
+    else if (v.ty == 16) box_of<T, 32, 16>(f, bw, bh);
+    else box_of<T, 32, 8>(f, bw, bh);
 }
 
 }  // namespace
@@ -968,6 +1004,28 @@ bool fused3d_variant_fits(int v, int esz) {
     // 64-wide FP64 tiles would hold one CTA per SM: not offered
     if (esz == 8 && kVariants[v].tx == 64) return false;
     return smem <= 227 * 1024;
+}
+
+// The 32x8 shape whose z-blocks take least time on this grid.  A z-block of zb planes is
+// zb + 1 steps; with b blocks to each of the 148 SMs a step of all of them takes about
+// 1.25 b + 1.6 us (fitted to FP64 and FP32 runs of 47x33x29 to 511^3: the first term is
+// the throughput of three or four resident CTAs, the second the latency of a step that
+// nothing else hides).  Short blocks pay the extra step, long ones leave SMs idle:
+// 259x193x125 FP64 measures 403, 273, 262, 285, 422 us at zb = 1, 8, 16, 32, 128 (the rule
+// takes 16), 127^3 walls 147, 117, 116, 138 at 1, 4, 8, 32 (8), 47x33x29 10, 16, 86 at
+// 1, 4, 32 (1), and 511^3 4.37 and 4.91 ms at 32 and 64 (32, the longest it considers).
+int fused3d_default_variant(const Geom &g) {
+    const double cols = (double)((g.n[0] + 32) / 32) * ((g.n[1] + 8) / 8);
+    int best = 0;
+    double cost = 0.0;
+    for (int v = 0; v < kNumVariants; v++) {
+        const Variant &w = kVariants[v];
+        if (w.tx != 32 || w.ty != 8 || w.cx * w.cy > 1 || w.trim || w.zb > 32) continue;
+        const double b = cols * ((g.n[2] + w.zb) / w.zb) / 148.0;
+        const double c = (w.zb + 1) * (1.25 * b + 1.6);
+        if (cost == 0.0 || c < cost) best = v, cost = c;
+    }
+    return best;
 }
 
 template <typename T>
@@ -997,20 +1055,21 @@ bool tma_encode(void *raw_base, int nd, const unsigned long long *dims, const un
 }
 
 // the 3D tensor map of input field f (map order) over a field allocation (raw
-// base, aligned) for a launch shape: box = one plane of the field's full box, or
-// of its trimmed box (stress fields of interior columns)
-bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int field, bool trimmed, void *map_out) {
+// base, aligned) for a launch shape: box = one plane of the field's box
+bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int field, void *map_out) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = get_encoder();
     if (!enc || variant < 0 || variant >= kNumVariants || field < 0 || field >= M_COUNT) return false;
     int bw = 0, bh = 0;
-    if (esz == 8) variant_box<double>(kVariants[variant], field, trimmed && field < kTrimmed, &bw, &bh);
-    else variant_box<float>(kVariants[variant], field, trimmed && field < kTrimmed, &bw, &bh);
+    if (esz == 8) variant_box<double>(kVariants[variant], field, &bw, &bh);
+    else variant_box<float>(kVariants[variant], field, &bw, &bh);
     cuuint64_t dims[3] = {(cuuint64_t)g.pitch, (cuuint64_t)g.rows, (cuuint64_t)g.planes};
     cuuint64_t strides[2] = {(cuuint64_t)(g.pitch * esz), (cuuint64_t)(g.sxy * esz)};
     cuuint32_t box[3] = {(cuuint32_t)bw, (cuuint32_t)bh, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    // L2 promotion of the box rows; FI_TMA_L2_PROMOTION=0/64/128/256 overrides
-    CUtensorMapL2promotion promo = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
+    // L2 promotion of the box rows: 64 bytes (511^3 FP64 4.35 ms against 4.49 at 256, whose
+    // wider fetches of a box's ring sectors raise the DRAM reads from 1.11 to 1.24 times the
+    // field bytes); FI_TMA_L2_PROMOTION=0/64/128/256 overrides
+    CUtensorMapL2promotion promo = CU_TENSOR_MAP_L2_PROMOTION_L2_64B;
     if (const char *e = getenv("FI_TMA_L2_PROMOTION")) {
         int v = atoi(e);
         promo = v == 0 ? CU_TENSOR_MAP_L2_PROMOTION_NONE
@@ -1024,15 +1083,14 @@ bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int
 }
 
 template <typename T>
-cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps18,
+cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
                            int variant, int *err, cudaStream_t s, int part_dim, int part) {
     if (variant < 0 || variant >= kNumVariants) variant = 0;
     const Variant v = kVariants[variant];
     if (!fused3d_variant_fits(variant, (int)sizeof(T))) return cudaErrorInvalidConfiguration;
-    const InMaps &mp = *reinterpret_cast<const InMaps *>(maps18);
+    const InMaps &mp = *reinterpret_cast<const InMaps *>(maps11);
     if (v.tx == 64) {
         if constexpr (sizeof(T) == 4) {
-            if (v.ty == 4) return launch_variant<T, 64, 4>(g, p, in, out, mp, v, err, s, part_dim, part);
             return launch_variant<T, 64, 8>(g, p, in, out, mp, v, err, s, part_dim, part);
         }
         return cudaErrorInvalidConfiguration;

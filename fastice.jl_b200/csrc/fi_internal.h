@@ -195,21 +195,22 @@ void bc_set_serial(const Geom &g, BcBatch &b);
 // P,tau,V read from `in`, written to `out`; eta read from in.eta, eta_next written.
 template <typename T>
 bool fused3d_supported(const Geom &g, const KParams &p, bool ib);
-// maps18: the eleven full-box input tensor maps (P, txx, tyy, tzz, txy, txz, tyz, Vx,
-// Vy, Vz, eta) then the trimmed-box maps of the seven stresses, 128 bytes each,
-// encoded with fused3d_encode_map for the variant
+// maps11: the input tensor maps (P, txx, tyy, tzz, txy, txz, tyz, Vx, Vy, Vz, eta), 128
+// bytes each, encoded with fused3d_encode_map for the variant
 // part_dim -1: every tile; 0 / 1: the tiles of the split faces along x / y (part 0)
 // or every other tile (part 1) -- the two halves of an iteration whose halo
 // exchange overlaps the second half
 template <typename T>
-cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps18,
+cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
                            int variant, int *err, cudaStream_t s, int part_dim = -1, int part = 0);
-// field: index in the map order above (0..10); trimmed: the interior box of a stress
-bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int field, bool trimmed, void *map_out);
+// field: index in the map order above (0..10)
+bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int field, void *map_out);
 // generic tiled tensor map (fi_fused3d.cu): nd dims, strides of dims 1..nd-1 in bytes
 bool tma_encode(void *raw_base, int nd, const unsigned long long *dims, const unsigned long long *strides,
                 const unsigned *box, int esz, void *map_out);
 int fused3d_num_variants();
+// the launch shape a model starts with, by its grid
+int fused3d_default_variant(const Geom &g);
 // launch shapes with the same key read through the same tensor maps
 int fused3d_variant_key(int v);
 // whether launch shape v fits a CTA in precision esz (8 or 4 bytes)

@@ -69,11 +69,8 @@ struct fi_model {
     cudaEvent_t ev_bnd = nullptr, ev_int = nullptr;
     bool interior_pending = false;  // stream2 work that `stream` has not waited for yet
     int split_begun = -1;           // split dimension of a begun iteration awaiting its second half
-    alignas(64) unsigned char pend_maps[18][128];
+    alignas(64) unsigned char pend_maps[11][128];
     unsigned char pend_ptrs[2][sizeof(fi::Ptrs<double>)];  // in / out of the begun iteration
-    // trimmed-box maps of the seven stress fields (interior columns of trimmed launch shapes)
-    alignas(64) unsigned char tmap_base[7][128];
-    alignas(64) unsigned char tmap_alt[7][128];
 
     bool is_f64() const { return d.dtype == FI_F64; }
 

@@ -244,8 +244,8 @@ fi_status fi_model_synchronize(fi_model *m);
 /* which kernel path the model runs (fi_path, never AUTO) */
 fi_status fi_model_path(const fi_model *m, int32_t *path);
 
-/* Launch shape of the fused sweep: tile width and height, z-block depth,
- * thread-block cluster shape and trimmed interior boxes.  A shape that does not
+/* Launch shape of the fused sweep: tile width and height, z-block depth and
+ * thread-block cluster shape; a model starts with one chosen by its grid.  A shape that does not
  * fit a CTA in the model's precision is rejected by fi_model_set_variant with
  * FI_ERR_UNSUPPORTED.  fi_model_autotune times every shape offered in the model's
  * precision for `iters` iterations on the model itself (so the model advances
