@@ -426,6 +426,27 @@ fi_status reference_pairs(fi_model *m, int pairs) {
     for (int q = 0; q < pairs; q++) FI_CHECK_CUDA(cudaGraphLaunch(m->pair_graph[e], m->stream), "graph launch");
     return FI_OK;
 }
+// Iterations of a 2D model by launches of several each (fi_tile2d.cu): an even number of
+// launches, so that the state ends in the buffers it started in, with η_next holding the
+// viscosity of the iteration before, as after the reference's swap.
+template <typename T>
+fi_status tile2d_advance(fi_model *m, int niter) {
+    const Tile2DPlan plan = tile2d_plan(m->g);
+    const int pairs = (niter + 2 * plan.k - 1) / (2 * plan.k), L = 2 * pairs;
+    for (int l = 0; l < L; l++) {
+        const int k = (int)((long long)niter * (l + 1) / L - (long long)niter * l / L);
+        Ptrs<T> a = m->ptrs<T>(false), b = m->ptrs<T>(true);
+        b.eta = (T *)m->eta_alt;
+        if (l & 1) std::swap(a, b);
+        if (m->kp.freeze_eta) a.eta = (T *)m->cur(FI_FIELD_ETA);
+        FI_CHECK_CUDA(launch_tile2d<T>(m->g, m->kp, a, b, (T *)m->cur(FI_FIELD_ETA_NEXT), plan.shape, k, l == L - 1, m->stream),
+                      "2D iterations");
+    }
+    m->alt_scratch = true;
+    m->iterations += niter;
+    return FI_OK;
+}
+
 constexpr int kPairGraphMin = 8;  // advances of at least this many iterations replay the graph
 
 template <typename T>
@@ -445,6 +466,18 @@ fi_status advance_t(fi_model *m, int niter) {
             }
             if (m->full_iters >= 2) m->kp.skip_zeros = 1;
         }
+    }
+    if (m->tile2d && niter >= 2) {
+        // a launch wraps around a periodic dimension: one ordinary iteration first makes the
+        // two ends agree if the state may have been written from outside
+        const bool per = m->kp.bc_kind[0][0] == FI_BC_PERIODIC || m->kp.bc_kind[1][0] == FI_BC_PERIODIC;
+        if (per && (m->full_iters == 0 || m->state_ptr_out)) {
+            if (fi_status st = reference_iteration<T>(m); st != FI_OK) return st;
+            m->iterations++;
+            m->full_iters++;
+            niter--;
+        }
+        if (niter >= 2) return tile2d_advance<T>(m, niter);
     }
     if (m->path != FI_PATH_FUSED && niter >= kPairGraphMin) {
         const int pairs = niter / 2;
@@ -545,14 +578,14 @@ BcBatch model_velocity_batch(const fi_model *m, int d) { return velocity_batch(m
 fi_status model_refresh_ibf(fi_model *m) { return m->is_f64() ? refresh_ibf<double>(m) : refresh_ibf<float>(m); }
 
 // Second state buffer of every state field, for drivers that double-buffer a
-// model whose own path updates in place (the batched 2D sweep); a new buffer
-// starts as a copy of the current state, ghosts included.
+// model whose own path updates in place (the batched 2D sweep); a new buffer, and one
+// that only served as scratch, starts as a copy of the current state, ghosts included.
 bool model_field_used(const fi_model *m, int f) { return field_used(m, f); }
 
 fi_status model_ensure_second_state(fi_model *m) {
     for (int f = 0; f < kState; f++) {
-        if (!field_used(m, f) || m->alt[f]) continue;
-        if (field_alloc(&m->alt[f], m->elems, m->esz) != cudaSuccess) {
+        if (!field_used(m, f) || (m->alt[f] && !m->alt_scratch)) continue;
+        if (!m->alt[f] && field_alloc(&m->alt[f], m->elems, m->esz) != cudaSuccess) {
             cudaGetLastError();
             set_error("device allocation failed (second state buffer)");
             return FI_ERR_OOM;
@@ -562,6 +595,7 @@ fi_status model_ensure_second_state(fi_model *m) {
         FI_CHECK_CUDA(cudaMemcpyAsync(dst, src, (m->elems + 64) * m->esz, cudaMemcpyDeviceToDevice, m->stream),
                       "second state buffer");
     }
+    m->alt_scratch = false;
     FI_CHECK_CUDA(cudaStreamSynchronize(m->stream), "second state buffer");
     return FI_OK;
 }
@@ -634,6 +668,31 @@ extern "C" {
 const char *fi_last_error(void) { return g_last_error.c_str(); }
 int fi_abi_version(void) { return FI_ABI_VERSION; }
 
+}  // extern "C"
+
+// The scratch buffers of a 2D model on the default path (fi_tile2d.cu) in one zero-filled
+// allocation: the second state and the third viscosity buffer.
+static fi_status alloc_scratch2d(fi_model *m) {
+    const size_t stride = ((m->elems + 64) * m->esz + 255) / 256 * 256;
+    size_t count = 1;
+    for (int f = 0; f < kState; f++) count += field_used(m, f) ? 1 : 0;
+    m->block_bytes = count * stride;
+    if (cudaMalloc(&m->block, m->block_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        m->block = nullptr;
+        return set_error("device allocation failed (" + std::to_string(m->block_bytes) + " bytes)"), FI_ERR_OOM;
+    }
+    FI_CHECK_CUDA(cudaMemsetAsync(m->block, 0, m->block_bytes, m->stream), "memset");
+    char *p = (char *)m->block + kXOff * m->esz;
+    for (int f = 0; f < kState; f++)
+        if (field_used(m, f)) m->alt[f] = p, p += stride;
+    m->eta_alt = p;
+    m->tile2d = m->alt_scratch = true;
+    return FI_OK;
+}
+
+extern "C" {
+
 fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
     if (!out) return set_error("null output handle"), FI_ERR_ARG;
     *out = nullptr;
@@ -696,6 +755,7 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
             }
 
     const size_t bytes = m->elems * m->esz;
+    if (gr.nd == 2 && desc->path == FI_PATH_AUTO && alloc_scratch2d(m) != FI_OK) return fail(FI_ERR_OOM);
     for (int f = 0; f < FI_FIELD_COUNT; f++) {
         if (!field_used(m, f) || is_residual(f)) continue;
         if (field_alloc(&m->base[f], m->elems, m->esz) != cudaSuccess) {
@@ -747,8 +807,13 @@ fi_status fi_model_destroy(fi_model *m) {
     cudaSetDevice(m->d.device);
     if (m->stream) cudaStreamSynchronize(m->stream);
     if (m->stream2) cudaStreamSynchronize(m->stream2);
-    for (int f = 0; f < FI_FIELD_COUNT; f++) field_free(m->base[f], m->esz);
-    for (int f = 0; f < kState; f++) field_free(m->alt[f], m->esz);
+    auto release = [&](void *p) {
+        const char *c = (const char *)p, *b = (const char *)m->block;
+        if (!(b && c >= b && c < b + m->block_bytes)) field_free(p, m->esz);
+    };
+    for (int f = 0; f < FI_FIELD_COUNT; f++) release(m->base[f]);
+    for (int f = 0; f < kState; f++) release(m->alt[f]);
+    if (m->block) cudaFree(m->block);
     if (m->d_err) cudaFree(m->d_err);
     if (m->d_ibf) cudaFree(m->d_ibf);
     if (m->d_blist) cudaFree(m->d_blist);

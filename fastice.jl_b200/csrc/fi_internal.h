@@ -217,6 +217,19 @@ int fused3d_variant_key(int v);
 bool fused3d_variant_fits(int v, int esz);
 const char *fused3d_variant_name(int v);
 
+// ---- several 2D iterations in one launch (fi_tile2d.cu) ----
+struct Tile2DPlan {
+    int shape;  // region shape
+    int k;      // most iterations of one launch
+};
+Tile2DPlan tile2d_plan(const Geom &g);
+// k iterations: P, τ, V, η read from `in`, written to `out` (distinct buffers, ghosts
+// included); with write_prev, η before the last of them to eta_prev (interior).  η is
+// read only when frozen.
+template <typename T>
+cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, T *eta_prev, int shape,
+                          int k, bool write_prev, cudaStream_t s);
+
 // ---- mixed-precision solve helpers (fi_mixed.cu) ----
 template <typename S, typename D>
 cudaError_t launch_convert(const S *src, D *dst, long long n, double scale, cudaStream_t s);

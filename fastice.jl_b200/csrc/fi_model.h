@@ -34,6 +34,13 @@ struct fi_model {
     int fused_variant = 0;
     int maps_key = -1;  // launch-shape key (fused3d_variant_key) the tensor maps were encoded for
     bool ib = false;
+    // 2D models on the default path: several iterations in one launch (fi_tile2d.cu), which
+    // reads one state buffer and writes the other; a third viscosity buffer beside η, η_next
+    bool tile2d = false;
+    bool alt_scratch = false;  // alt[] holds nothing of the model's state
+    void *eta_alt = nullptr;
+    void *block = nullptr;  // the allocation that holds both
+    size_t block_bytes = 0;
     long long iterations = 0;
     int *d_err = nullptr;  // device error word written by bounded waits
     unsigned char *d_ibf = nullptr;  // immersed-boundary activity byte per grid index (IbFlag bits)

@@ -60,10 +60,11 @@ class SolveRequest:
 
 
 def footprint_2d(n, esz: int) -> int:
-    """Device bytes of a batched 2D member: 15 state-sized arrays (P, τ×3, V×2 in
-    two buffers, η, η_next, the rheology's η field), rows padded to 32."""
+    """Device bytes of a batched 2D member: 16 state-sized arrays (P, τ×3, V×2 in
+    two buffers, η, η_next and a third viscosity buffer, the rheology's η field), rows
+    padded to 32."""
     pitch = ((31 + n[0] + 3 + 31) // 32) * 32
-    return 15 * pitch * (n[1] + 3) * esz + 4096
+    return 16 * pitch * (n[1] + 3) * esz + 4096
 
 
 def footprint_3d_ib(n, esz: int) -> int:

@@ -105,7 +105,9 @@ typedef struct {
 
 /* kernel-path selection (fi_model_desc.path) */
 typedef enum {
-    FI_PATH_AUTO = 0,      /* fused single-pass sweep where supported, else reference-shaped */
+    FI_PATH_AUTO = 0,      /* fused single-pass sweep where supported, else reference-shaped
+                              (2D: several iterations per launch, same results; reported as
+                              reference-shaped) */
     FI_PATH_REFERENCE = 1, /* reference-shaped: update_sigma, BC batch, update_V, BC batch */
     FI_PATH_FUSED = 2      /* fused sweep; FI_ERR_UNSUPPORTED if the problem is not covered */
 } fi_path;
