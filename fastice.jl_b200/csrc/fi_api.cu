@@ -369,6 +369,18 @@ fi_status refresh_ibf(fi_model *m) {
         FI_CHECK_CUDA(cudaMemcpy(m->d_blist, ids.data(), cnt * sizeof(uint2), cudaMemcpyHostToDevice), "block list");
     }
     m->n_blist = cnt;
+    if (m->ib_fused) {
+        FI_CHECK_CUDA(ib_runs(m->g, m->d_ibf, &m->ib_runs, m->stream), "active columns");
+        std::vector<int4> jobs;
+        ib_make_jobs(m->ib_runs, ib_job_depth({&m->ib_runs}), 0, &jobs);
+        m->ib_gen++;
+        if (m->d_jobs) cudaFree(m->d_jobs);
+        m->d_jobs = nullptr, m->n_jobs = (int)jobs.size();
+        if (m->n_jobs > 0) {
+            FI_CHECK_CUDA(cudaMalloc(&m->d_jobs, jobs.size() * sizeof(int4)), "jobs");
+            FI_CHECK_CUDA(cudaMemcpy(m->d_jobs, jobs.data(), jobs.size() * sizeof(int4), cudaMemcpyHostToDevice), "jobs");
+        }
+    }
     // captured iteration pairs hold the old list's launch size
     for (cudaGraphExec_t &g : m->pair_graph)
         if (g) cudaGraphExecDestroy(g), g = nullptr;
@@ -380,6 +392,7 @@ fi_status refresh_ibf(fi_model *m) {
 template <typename T>
 fi_status reference_iteration(fi_model *m) {
     Ptrs<T> f = m->ptrs<T>();
+    m->ib_synced = false;  // the other state buffer falls behind
     // once zeros hold, only the blocks with an active or a boundary point run
     const BlockList bl{m->d_blist, m->n_blist};
     // (a relaxed viscosity moves towards its target at every point, so it runs all)
@@ -449,6 +462,21 @@ fi_status tile2d_advance(fi_model *m, int niter) {
 
 constexpr int kPairGraphMin = 8;  // advances of at least this many iterations replay the graph
 
+// niter fused sweeps of an immersed-boundary model whose buffers agree
+template <typename T>
+fi_status fusedib_advance(fi_model *m, int niter) {
+    alignas(64) unsigned char maps[11][128];
+    for (int it = 0; it < niter; it++) {
+        const Ptrs<T> in = m->ptrs<T>(false), out = m->ptrs<T>(true);
+        model_ib_maps(m, maps);
+        FI_CHECK_CUDA(launch_fusedib<T>(m->g, m->kp, in, out, maps, m->d_jobs, m->n_jobs, m->d_err, m->stream),
+                      "fused immersed-boundary sweep");
+        m->parity ^= 1;
+        if (!m->kp.freeze_eta) m->eta_swapped = !m->eta_swapped;
+        m->iterations++;
+    }
+    return FI_OK;
+}
 template <typename T>
 fi_status advance_t(fi_model *m, int niter) {
     if (fi_status st = refresh_ibf<T>(m); st != FI_OK) return st;
@@ -457,6 +485,7 @@ fi_status advance_t(fi_model *m, int niter) {
         // ones skip the zeros of the inactive strict interior and the blocks outside
         // the block list
         m->kp.skip_zeros = 0;
+        if (m->full_iters < 2) m->ib_synced = false;
         if (!m->state_ptr_out) {
             while (m->full_iters < 2 && niter > 0) {
                 if (fi_status st = reference_iteration<T>(m); st != FI_OK) return st;
@@ -465,6 +494,10 @@ fi_status advance_t(fi_model *m, int niter) {
                 m->full_iters++;
             }
             if (m->full_iters >= 2) m->kp.skip_zeros = 1;
+        }
+        if (niter > 0 && model_ib_takes_fused(m, niter)) {
+            if (fi_status st = model_ib_sync(m); st != FI_OK) return st;
+            return fusedib_advance<T>(m, niter);
         }
     }
     if (m->tile2d && niter >= 2) {
@@ -550,6 +583,7 @@ fi_status norms_t(fi_model *m, double *out) {
 
 template <typename T>
 fi_status apply_bcs_t(fi_model *m) {
+    m->ib_synced = false;
     fi_status st = run_batch<T>(m, stress_batch);
     if (st == FI_OK) st = run_batch<T>(m, velocity_batch);
     if (st == FI_OK) st = run_eta_batch<T>(m, FI_FIELD_ETA);
@@ -572,6 +606,29 @@ bool fused_ok(const fi_model *m) {
 }
 
 }  // namespace
+
+// Two full iterations since anything else wrote the state, no state pointer handed out and
+// a viscosity that does not move away from the ice: points outside the jobs hold what they
+// will always hold.  Fewer iterations than kIbSyncMin are not worth the copy of the state.
+constexpr int kIbSyncMin = 6;
+bool model_ib_takes_fused(const fi_model *m, int niter) {
+    const bool eta_moves = !m->kp.freeze_eta && m->kp.rheo_relax != FI_RELAX_NONE;
+    return m->ib_fused && !m->state_ptr_out && m->full_iters >= 2 && !m->ibf_stale && !eta_moves &&
+           (m->ib_synced || niter >= kIbSyncMin);
+}
+void model_ib_maps(const fi_model *m, unsigned char (*maps)[128]) {
+    for (int f = 0; f < kState; f++) std::memcpy(maps[f], m->parity ? m->map_alt[f] : m->map_base[f], 128);
+    std::memcpy(maps[10], m->map_eta[m->eta_swapped ? 1 : 0], 128);
+}
+fi_status model_ib_sync(fi_model *m) {
+    if (m->ib_synced) return FI_OK;
+    for (int f = 0; f < kState; f++)
+        FI_CHECK_CUDA(cudaMemcpyAsync(field_raw(m->nxt(f), m->esz), field_raw(m->cur(f), m->esz), (m->elems + 64) * m->esz,
+                                      cudaMemcpyDeviceToDevice, m->stream),
+                      "second state buffer");
+    m->ib_synced = true;
+    return FI_OK;
+}
 
 BcBatch model_stress_batch(const fi_model *m, int d) { return stress_batch(m, d); }
 BcBatch model_velocity_batch(const fi_model *m, int d) { return velocity_batch(m, d); }
@@ -670,11 +727,11 @@ int fi_abi_version(void) { return FI_ABI_VERSION; }
 
 }  // extern "C"
 
-// The scratch buffers of a 2D model on the default path (fi_tile2d.cu) in one zero-filled
-// allocation: the second state and the third viscosity buffer.
-static fi_status alloc_scratch2d(fi_model *m) {
+// The second state buffer of a model whose default path needs one (and, in 2D, the third
+// viscosity buffer of fi_tile2d.cu), zero-filled, in one allocation.
+static fi_status alloc_second_state(fi_model *m) {
     const size_t stride = ((m->elems + 64) * m->esz + 255) / 256 * 256;
-    size_t count = 1;
+    size_t count = m->d.grid.nd == 2 ? 1 : 0;
     for (int f = 0; f < kState; f++) count += field_used(m, f) ? 1 : 0;
     m->block_bytes = count * stride;
     if (cudaMalloc(&m->block, m->block_bytes) != cudaSuccess) {
@@ -686,8 +743,8 @@ static fi_status alloc_scratch2d(fi_model *m) {
     char *p = (char *)m->block + kXOff * m->esz;
     for (int f = 0; f < kState; f++)
         if (field_used(m, f)) m->alt[f] = p, p += stride;
-    m->eta_alt = p;
-    m->tile2d = m->alt_scratch = true;
+    if (m->d.grid.nd == 2) m->eta_alt = p;
+    m->alt_scratch = m->d.grid.nd == 2;
     return FI_OK;
 }
 
@@ -755,7 +812,10 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
             }
 
     const size_t bytes = m->elems * m->esz;
-    if (gr.nd == 2 && desc->path == FI_PATH_AUTO && alloc_scratch2d(m) != FI_OK) return fail(FI_ERR_OOM);
+    if (gr.nd == 2 && desc->path == FI_PATH_AUTO) {
+        if (fi_status s = alloc_second_state(m); s != FI_OK) return fail(s);
+        m->tile2d = true;
+    }
     for (int f = 0; f < FI_FIELD_COUNT; f++) {
         if (!field_used(m, f) || is_residual(f)) continue;
         if (field_alloc(&m->base[f], m->elems, m->esz) != cudaSuccess) {
@@ -784,6 +844,15 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
                   cudaMalloc(&m->d_bcount, sizeof(int)) != cudaSuccess))
         return fail(cuda_fail(cudaGetLastError(), "activity bytes"));
     cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream);
+    bool away = false;  // a side whose values come from elsewhere
+    for (int k = 0; k < gr.nd; k++)
+        for (const fi_bc &side : desc->bc[k]) away = away || side.kind == FI_BC_PERIODIC || side.kind == FI_BC_HALO;
+    if (m->ib && desc->path == FI_PATH_AUTO && !away && alloc_second_state(m) == FI_OK) {
+        // (without room for it the model keeps the in-place iterations)
+        fi_status es = encode_maps(m);
+        if (es != FI_OK) return fail(es);
+        m->ib_fused = true;
+    }
     if (m->path == FI_PATH_FUSED) {
         m->fused_variant = fused3d_default_variant(g);
         fi_status es = encode_maps(m);
@@ -818,6 +887,7 @@ fi_status fi_model_destroy(fi_model *m) {
     if (m->d_ibf) cudaFree(m->d_ibf);
     if (m->d_blist) cudaFree(m->d_blist);
     if (m->d_bcount) cudaFree(m->d_bcount);
+    if (m->d_jobs) cudaFree(m->d_jobs);
     for (cudaGraphExec_t &g : m->pair_graph)
         if (g) cudaGraphExecDestroy(g);
     field_free(m->fP, m->esz);

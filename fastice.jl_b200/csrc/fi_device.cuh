@@ -97,6 +97,54 @@ __device__ __forceinline__ T third(T x) {
 #endif
 }
 
+// Sums of products with the rounding spelled out.  Left to the compiler, which product of a
+// sum goes into the fused multiply-add differs from kernel to kernel (and with the precision);
+// sweeps that take over from the in-place kernels of fi_reference.cu during a solve use the
+// forms those come out as, so that a model's values do not depend on the grouping of its
+// iterations.  FI_EXACT_ORDER builds round every product and sum, as the oracle.
+#ifdef FI_EXACT_ORDER
+template <typename T>
+__device__ __forceinline__ T mul_r(T a, T b) { return a * b; }
+template <typename T>
+__device__ __forceinline__ T fma_r(T a, T b, T c) { return a * b + c; }
+#else
+__device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
+#endif
+// wa a - wb b
+template <typename T>
+__device__ __forceinline__ T diff_r(T wa, T a, T wb, T b) { return fma_r(wa, a, -mul_r(wb, b)); }
+// a i + b j
+template <typename T>
+__device__ __forceinline__ T sum_r(T a, T i, T b, T j) { return fma_r(a, i, mul_r(b, j)); }
+// o - (o - e r) dt
+template <typename T>
+__device__ __forceinline__ T relax_r(T o, T e, T r, T dt) { return fma_r(-fma_r(-e, r, o), dt, o); }
+// The divergence of the differences s0, s1 (, s2) over the spacings 1/i and the deviators of
+// their rates (ND 2: d[2] is not set)
+template <int ND, typename T>
+__device__ __forceinline__ T rates_r(const T (&s)[3], const T *i, T (&d)[3]) {
+    const T e0 = mul_r(s[0], i[0]), e1 = mul_r(s[1], i[1]), e2 = ND == 3 ? mul_r(s[2], i[2]) : T(0);
+#ifdef FI_EXACT_ORDER
+    const T v = ND == 3 ? e0 + e1 + e2 : e0 + e1, t = third(v);
+    d[0] = e0 - t, d[1] = e1 - t, d[2] = e2 - t;
+#else
+    T v;
+    if (sizeof(T) == 8) {
+        v = fma_r(s[0], i[0], e1);
+        if (ND == 3) v = fma_r(s[2], i[2], v);
+        const T t = mul_r(v, T(1.0 / 3.0));
+        d[0] = fma_r(s[0], i[0], -t), d[1] = e1 - t, d[2] = ND == 3 ? fma_r(s[2], i[2], -t) : T(0);
+    } else {
+        v = ND == 3 ? e0 + e1 + e2 : e0 + e1;
+        d[0] = fma_r(-v, T(1.0 / 3.0), e0), d[1] = fma_r(-v, T(1.0 / 3.0), e1), d[2] = fma_r(-v, T(1.0 / 3.0), e2);
+    }
+#endif
+    return v;
+}
+
 // η_next from τII² = s2 (rheology(τII) with τII = sqrt(s2)).  Production builds
 // evaluate Glen's law with the integer exponent n = 3 as 0.5/(A s2) and its
 // viscoplastic regularisation as 1/(2 A s2 + 1/η_reg): the same function without

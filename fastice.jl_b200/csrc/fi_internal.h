@@ -95,8 +95,12 @@ struct Ptrs {
 };
 // bits of the precomputed immersed-boundary activity byte: update_σ! points
 // (isvalid(na) && !isempty(ns)) at ccc, vvc, vcv, cvv and update_V! points
-// (isvalid(ns) && !isempty(na)) at vcc, cvc, ccv
-enum IbFlag { IBF_S_CCC = 1, IBF_S_VVC = 2, IBF_S_VCV = 4, IBF_S_CVV = 8, IBF_V_VCC = 16, IBF_V_CVC = 32, IBF_V_CCV = 64 };
+// (isvalid(ns) && !isempty(na)) at vcc, cvc, ccv; FULL: all seven, and every volume
+// fraction that the updates of the index read is exactly 1 (set in precomputed bytes only)
+enum IbFlag {
+    IBF_S_CCC = 1, IBF_S_VVC = 2, IBF_S_VCV = 4, IBF_S_CVV = 8, IBF_V_VCC = 16, IBF_V_CVC = 32, IBF_V_CCV = 64,
+    IBF_FULL = 128
+};
 
 // one boundary-condition operation on a face (see kernel bc_dim_kernel)
 enum BcOp { BC_DIRICHLET = 0, BC_NEUMANN = 1, BC_PERIODIC = 2 };

@@ -3,6 +3,7 @@
 // fi_batch.cu).
 #pragma once
 
+#include "fi_fusedib.h"
 #include "fi_internal.h"
 
 namespace fi {
@@ -60,6 +61,14 @@ struct fi_model {
     // a caller ends both for good.
     int full_iters = 0;
     bool state_ptr_out = false;
+    // Immersed-boundary models on the default path: the fused sweep (fi_fusedib.cu) reads one
+    // state buffer and writes the other, once both agree outside its jobs (ib_synced: since
+    // the last two full iterations nothing but it wrote the state)
+    bool ib_fused = false, ib_synced = false;
+    std::vector<fi::IbRun> ib_runs;
+    unsigned long long ib_gen = 0;  // times the runs were made
+    int4 *d_jobs = nullptr;
+    int n_jobs = 0;
     void *fP = nullptr;    // pressure forcing (defect-correction shadow models only)
     void *d_stage = nullptr;  // staging buffer of set_field (contiguous rows of host data)
     size_t stage_bytes = 0;
@@ -137,6 +146,12 @@ fi_status mixed_phase_a_end(fi_model *m);
 fi_status mixed_picard(fi_model *m);
 fi_status mixed_correction_begin(fi_model *m);
 fi_status mixed_correction_end(fi_model *m);
+// whether an immersed-boundary model's next niter iterations are the fused sweep, the copy
+// that makes its two state buffers agree, and the tensor maps of what the sweep reads
+// (fi_api.cu)
+bool model_ib_takes_fused(const fi_model *m, int niter);
+fi_status model_ib_sync(fi_model *m);
+void model_ib_maps(const fi_model *m, unsigned char (*maps)[128]);
 // the boundary batches of the reference-shaped iteration (fi_api.cu) and the refresh of
 // an immersed-boundary model's activity bytes and block list when stale
 fi::BcBatch model_stress_batch(const fi_model *m, int d);

@@ -927,14 +927,26 @@ cudaError_t launch_compute_residuals(const Geom &g, const KParams &p, const Ptrs
 }
 
 // activity bytes over the vertex range (null_spaces.jl:41-43 at the seven
-// locations the masked kernels test)
+// locations the masked kernels test; FULL where every fraction they read is 1)
 template <typename T>
 __global__ void __launch_bounds__(256) ib_flags_kernel(Geom g, KParams p, Ptrs<T> f, unsigned char *flags) {
     Idx x = vertex_index(g);
     if (!x.ok) return;
     Ptrs<T> q = f;
     q.ibf = nullptr;
-    flags[x.I] = (unsigned char)ib_flags_at(q, x.I, g.pitch, g.sxy, T(p.small));
+    const long long I = x.I, sx = g.pitch, sxy = g.sxy;
+    unsigned b = ib_flags_at(q, I, sx, sxy, T(p.small));
+    if (b == 0x7fu) {
+        const T *c = f.wna[W_CCC], *xy = f.wna[W_VVC], *xz = f.wna[W_VCV], *yz = f.wna[W_CVV];
+        const T *nx = f.wns[W_VCC], *ny = f.wns[W_CVC], *nz = f.wns[W_CCV];
+        const T w[] = {c[I], c[I - 1], c[I - sx], c[I - sxy], xy[I], xy[I + sx], xy[I + 1], xz[I], xz[I + sxy], xz[I + 1],
+                       yz[I], yz[I + sxy], yz[I + sx], nx[I], nx[I + 1], nx[I - sx], nx[I - sxy], ny[I], ny[I + sx],
+                       ny[I - 1], ny[I - sxy], nz[I], nz[I + sxy], nz[I - 1], nz[I - sx]};
+        bool one = true;
+        for (const T v : w) one = one && v == T(1);
+        if (one) b |= IBF_FULL;
+    }
+    flags[I] = (unsigned char)b;
 }
 
 template <typename T>

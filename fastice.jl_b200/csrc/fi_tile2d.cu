@@ -102,16 +102,16 @@ __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, co
             const T el = sE[a - 1];
             etl[r] = el;
             etd[r] = ed;
-            const T exx = (sVx[a + 1] - v.vx[r]) * idx;
-            const T eyy = (vyu - v.vy[r]) * idy;
-            const T exy = T(0.5) * ((v.vy[r] - sVy[a - 1]) * idx + (v.vx[r] - vxd) * idy);
-            const T divV = exx + eyy;
+            const T s[3] = {sVx[a + 1] - v.vx[r], vyu - v.vy[r], T(0)};
+            T d[3];
+            const T divV = rates_r<2>(s, q.inv_dx, d);
+            const T exy = h(sum_r(v.vy[r] - sVy[a - 1], idx, v.vx[r] - vxd, idy));
             const T dv = forced ? divV + __ldg(in.fP + v.at[r]) : divV;
-            const T nP = v.P[r] - dv * v.et[r] * q.dt_P;
-            const T nxx = v.xx[r] - (v.xx[r] - T(2.0) * v.et[r] * (exx - third(divV))) * q.dt_tau[0];
-            const T nyy = v.yy[r] - (v.yy[r] - T(2.0) * v.et[r] * (eyy - third(divV))) * q.dt_tau[1];
+            const T nP = fma_r(-mul_r(dv, v.et[r]), q.dt_P, v.P[r]);
+            const T nxx = relax_r(v.xx[r], T(2.0) * v.et[r], d[0], q.dt_tau[0]);
+            const T nyy = relax_r(v.yy[r], T(2.0) * v.et[r], d[1], q.dt_tau[1]);
             const T e_xy = h(h(edl + ed) + h(el + v.et[r]));
-            T nxy = v.xy[r] - (v.xy[r] - T(2.0) * e_xy * exy) * q.dt_tau[3];
+            T nxy = relax_r(v.xy[r], T(2.0) * e_xy, exy, q.dt_tau[3]);
             vxd = v.vx[r];
             ed = v.et[r];
             edl = el;
@@ -159,19 +159,17 @@ __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, co
             const int a = a0 + r * PW;
             const T xyu = r + 1 < PY ? v.xy[r + 1] : sXY[a + PW];
             const T xyru = sXY[a + PW + 1];
-            T nvx = v.vx[r] + div_fast(-(v.P[r] - sP[a - 1]) * idx + (v.xx[r] - sXX[a - 1]) * idx + (xyu - v.xy[r]) * idy - (GF ? v.gx[r] : q.g_val[0]),
-                                       h(etl[r] + v.et[r])) *
-                                  q.dt_V[0];
-            T nvy = v.vy[r] + div_fast(-(v.P[r] - Pd) * idy + (v.yy[r] - yyd) * idy + (xyr - v.xy[r]) * idx - (GF ? v.gy[r] : q.g_val[1]),
-                                       h(etd[r] + v.et[r])) *
-                                  q.dt_V[1];
+            const T fx = fma_r(xyu - v.xy[r], idy, sum_r(v.xx[r] - sXX[a - 1], idx, -(v.P[r] - sP[a - 1]), idx));
+            const T fy = fma_r(xyr - v.xy[r], idx, sum_r(v.yy[r] - yyd, idy, -(v.P[r] - Pd), idy));
+            T nvx = fma_r(div_fast(fx - (GF ? v.gx[r] : q.g_val[0]), h(etl[r] + v.et[r])), q.dt_V[0], v.vx[r]);
+            T nvy = fma_r(div_fast(fy - (GF ? v.gy[r] : q.g_val[1]), h(etd[r] + v.et[r])), q.dt_V[1], v.vy[r]);
             T ne = v.et[r];
             if (!frozen) {
                 if (linear) {
                     ne = p.rheo_eta_is_field ? __ldg(in.eta_lin + v.at[r]) : T(p.rheo_eta);
                 } else {
                     const T lxy = h(h(v.xy[r] + xyr) + h(xyu + xyru));
-                    const T s2 = T(0.5) * (v.xx[r] * v.xx[r] + v.yy[r] * v.yy[r]) + lxy * lxy;
+                    const T s2 = h(sum_r(v.xx[r], v.xx[r], v.yy[r], v.yy[r])) + mul_r(lxy, lxy);
                     ne = rheology_s2(p, q.rheo_A, q.rheo_inv_eta_reg, in.eta_lin, in.A, v.et[r], (long long)v.at[r], s2);
                 }
             }

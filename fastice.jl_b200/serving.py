@@ -68,10 +68,10 @@ def footprint_2d(n, esz: int) -> int:
 
 
 def footprint_3d_ib(n, esz: int) -> int:
-    """Device bytes of a 3D immersed-boundary model: 10 state fields, η, η_next,
-    16 volume fractions, 4 residual fields, rows padded to 32."""
+    """Device bytes of a 3D immersed-boundary model: 10 state fields in two buffers, η,
+    η_next, 16 volume fractions, 4 residual fields, rows padded to 32."""
     pitch = ((31 + n[0] + 3 + 31) // 32) * 32
-    return 30 * pitch * (n[1] + 3) * (n[2] + 3) * esz + (1 << 20)
+    return 40 * pitch * (n[1] + 3) * (n[2] + 3) * esz + (1 << 20)
 
 
 def rel_measure_3d(norms: np.ndarray, rho_g_inf: float, length_z: float) -> float:
