@@ -469,7 +469,7 @@ fi_status fusedib_advance(fi_model *m, int niter) {
     for (int it = 0; it < niter; it++) {
         const Ptrs<T> in = m->ptrs<T>(false), out = m->ptrs<T>(true);
         model_ib_maps(m, maps);
-        FI_CHECK_CUDA(launch_fusedib<T>(m->g, m->kp, in, out, maps, m->d_jobs, m->n_jobs, m->d_err, m->stream),
+        FI_CHECK_CUDA(launch_fusedib<T>(m->g, m->kp, in, out, maps, m->d_jobs, m->n_jobs, m->d_err, m->stream, it > 0),
                       "fused immersed-boundary sweep");
         m->parity ^= 1;
         if (!m->kp.freeze_eta) m->eta_swapped = !m->eta_swapped;
@@ -527,7 +527,7 @@ fi_status advance_t(fi_model *m, int niter) {
             alignas(64) unsigned char maps[11][128];
             for (int f = 0; f < kState; f++) std::memcpy(maps[f], m->parity ? m->map_alt[f] : m->map_base[f], 128);
             std::memcpy(maps[10], m->map_eta[m->eta_swapped ? 1 : 0], 128);
-            FI_CHECK_CUDA(launch_fused3d<T>(m->g, m->kp, in, out, maps, m->fused_variant, m->d_err, m->stream),
+            FI_CHECK_CUDA(launch_fused3d<T>(m->g, m->kp, in, out, maps, m->fused_variant, m->d_err, m->stream, -1, 0, it > 0),
                           "fused sweep");
             m->parity ^= 1;
             if (!m->kp.freeze_eta) m->eta_swapped = !m->eta_swapped;

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(Layout<T, TX, TY>::NT, Layout<T, TX, TY>::MINB
     __syncthreads();
     Ctx<T, TX, TY> c;
     init_ctx(c, g, p, smem_raw, zb, tm);
+    chain_launches();
     // Interior columns need no range tests, no x or y boundary values and no images, but in
     // FP64 a body of their own costs more in instruction fetches than it saves (259x193x125:
     // 268 us an iteration with it, 251 without; 511^3 4.37 and 4.26 ms).  FP32 code is
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(Layout<T, TX, TY>::NT, Layout<T, TX, TY>::MINB
 
 template <typename T, int TX, int TY>
 cudaError_t launch_variant(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const InMaps &maps,
-                           Variant v, int *err, cudaStream_t s, int part_dim, int part) {
+                           Variant v, int *err, cudaStream_t s, int part_dim, int part, bool chained) {
     using Lay = Layout<T, TX, TY>;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -205,6 +206,11 @@ cudaError_t launch_variant(const Geom &g, const KParams &p, const Ptrs<T> &in, c
         attr[0].val.clusterDim.x = v.cx;
         attr[0].val.clusterDim.y = v.cy;
         attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    } else if (chained) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
@@ -361,29 +367,29 @@ bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int
 
 template <typename T>
 cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
-                           int variant, int *err, cudaStream_t s, int part_dim, int part) {
+                           int variant, int *err, cudaStream_t s, int part_dim, int part, bool chained) {
     if (variant < 0 || variant >= kNumVariants) variant = 0;
     const Variant v = kVariants[variant];
     if (!fused3d_variant_fits(variant, (int)sizeof(T))) return cudaErrorInvalidConfiguration;
     const InMaps &mp = *reinterpret_cast<const InMaps *>(maps11);
     if (v.tx == 64) {
         if constexpr (sizeof(T) == 4) {
-            return launch_variant<T, 64, 8>(g, p, in, out, mp, v, err, s, part_dim, part);
+            return launch_variant<T, 64, 8>(g, p, in, out, mp, v, err, s, part_dim, part, chained);
         }
         return cudaErrorInvalidConfiguration;
     }
     switch (v.ty) {
-        case 4: return launch_variant<T, 32, 4>(g, p, in, out, mp, v, err, s, part_dim, part);
-        case 16: return launch_variant<T, 32, 16>(g, p, in, out, mp, v, err, s, part_dim, part);
-        default: return launch_variant<T, 32, 8>(g, p, in, out, mp, v, err, s, part_dim, part);
+        case 4: return launch_variant<T, 32, 4>(g, p, in, out, mp, v, err, s, part_dim, part, chained);
+        case 16: return launch_variant<T, 32, 16>(g, p, in, out, mp, v, err, s, part_dim, part, chained);
+        default: return launch_variant<T, 32, 8>(g, p, in, out, mp, v, err, s, part_dim, part, chained);
     }
 }
 
 template bool fused3d_supported<double>(const Geom &, const KParams &, bool);
 template bool fused3d_supported<float>(const Geom &, const KParams &, bool);
 template cudaError_t launch_fused3d<double>(const Geom &, const KParams &, const Ptrs<double> &, const Ptrs<double> &,
-                                            const void *, int, int *, cudaStream_t, int, int);
+                                            const void *, int, int *, cudaStream_t, int, int, bool);
 template cudaError_t launch_fused3d<float>(const Geom &, const KParams &, const Ptrs<float> &, const Ptrs<float> &,
-                                           const void *, int, int *, cudaStream_t, int, int);
+                                           const void *, int, int *, cudaStream_t, int, int, bool);
 
 }  // namespace fi

@@ -347,6 +347,7 @@ __device__ __forceinline__ void run_job(const Geom &g, const KParams &p, const T
     c.sx = g.pitch;
     c.sxy = g.sxy;
     c.hx0 = c.hx1 = c.hy0 = c.hy1 = false;
+    chain_launches();
     sweep_ib(c, p, q, in, out, maps, bars, released, err);
 }
 
@@ -401,6 +402,20 @@ cudaError_t lift_smem() {
                 : cudaFuncSetAttribute(fusedib_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess && dev < 64) set[dev] = true;
     return e;
+}
+
+template <typename T>
+cudaLaunchConfig_t launch_config(int blocks, cudaStream_t s, bool chained, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(Layout<T, IX, IY>::NT);
+    cfg.dynamicSmemBytes = Layout<T, IX, IY>::SMEM;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cfg;
 }
 
 }  // namespace
@@ -461,28 +476,28 @@ void ib_make_jobs(const std::vector<IbRun> &runs, int zb, int member, std::vecto
 
 template <typename T>
 cudaError_t launch_fusedib(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
-                           const int4 *jobs, int njobs, int *err, cudaStream_t s) {
-    using Lay = Layout<T, IX, IY>;
+                           const int4 *jobs, int njobs, int *err, cudaStream_t s, bool chained) {
     if (njobs <= 0) return cudaSuccess;
     if (cudaError_t r = lift_smem<T, false>(); r != cudaSuccess) return r;
-    fusedib_kernel<T><<<njobs, Lay::NT, Lay::SMEM, s>>>(g, p, make_tconst<T>(p), in, out,
-                                                        *reinterpret_cast<const InMaps *>(maps11), jobs, err);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = launch_config<T>(njobs, s, chained, attr);
+    return cudaLaunchKernelEx(&cfg, fusedib_kernel<T>, g, p, make_tconst<T>(p), in, out, *reinterpret_cast<const InMaps *>(maps11),
+                              jobs, err);
 }
 
 template <typename T>
-cudaError_t launch_fusedib_batched(const IbFusedMember<T> *members, const int4 *jobs, int njobs, int e, cudaStream_t s) {
-    using Lay = Layout<T, IX, IY>;
+cudaError_t launch_fusedib_batched(const IbFusedMember<T> *members, const int4 *jobs, int njobs, int e, cudaStream_t s, bool chained) {
     if (njobs <= 0) return cudaSuccess;
     if (cudaError_t r = lift_smem<T, true>(); r != cudaSuccess) return r;
-    fusedib_batched<T><<<njobs, Lay::NT, Lay::SMEM, s>>>(members, jobs, e);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = launch_config<T>(njobs, s, chained, attr);
+    return cudaLaunchKernelEx(&cfg, fusedib_batched<T>, members, jobs, e);
 }
 
 #define FI_INST(T)                                                                                                     \
     template cudaError_t launch_fusedib<T>(const Geom &, const KParams &, const Ptrs<T> &, const Ptrs<T> &, const void *, \
-                                           const int4 *, int, int *, cudaStream_t);                                  \
-    template cudaError_t launch_fusedib_batched<T>(const IbFusedMember<T> *, const int4 *, int, int, cudaStream_t);
+                                           const int4 *, int, int *, cudaStream_t, bool);                                  \
+    template cudaError_t launch_fusedib_batched<T>(const IbFusedMember<T> *, const int4 *, int, int, cudaStream_t, bool);
 FI_INST(double)
 FI_INST(float)
 #undef FI_INST

@@ -34,10 +34,11 @@ cudaError_t ib_runs(const Geom &g, const unsigned char *flags, std::vector<IbRun
 int ib_job_depth(const std::vector<const std::vector<IbRun> *> &all);
 void ib_make_jobs(const std::vector<IbRun> &runs, int zb, int member, std::vector<int4> *jobs);
 
+// (chained: right after another of these launches on the stream)
 template <typename T>
 cudaError_t launch_fusedib(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
-                           const int4 *jobs, int njobs, int *err, cudaStream_t s);
+                           const int4 *jobs, int njobs, int *err, cudaStream_t s, bool chained);
 template <typename T>
-cudaError_t launch_fusedib_batched(const IbFusedMember<T> *members, const int4 *jobs, int njobs, int e, cudaStream_t s);
+cudaError_t launch_fusedib_batched(const IbFusedMember<T> *members, const int4 *jobs, int njobs, int e, cudaStream_t s, bool chained);
 
 }  // namespace fi

@@ -327,7 +327,7 @@ fi_status advance_fused(fi_ib_batch *b, const std::vector<fi_model *> &fused, in
     }
     for (int it = 0; it < niter; it++, e ^= 1)
         FB_CHECK(launch_fusedib_batched<T>(reinterpret_cast<const IbFusedMember<T> *>(b->d_fused), b->d_jobs, b->njobs, e,
-                                           b->stream),
+                                           b->stream, it > 0),
                  "shared fused sweep");
     for (fi_model *m : fused) {
         m->iterations += niter;

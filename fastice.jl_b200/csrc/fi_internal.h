@@ -206,7 +206,7 @@ bool fused3d_supported(const Geom &g, const KParams &p, bool ib);
 // exchange overlaps the second half
 template <typename T>
 cudaError_t launch_fused3d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, const void *maps11,
-                           int variant, int *err, cudaStream_t s, int part_dim = -1, int part = 0);
+                           int variant, int *err, cudaStream_t s, int part_dim = -1, int part = 0, bool chained = false);
 // field: index in the map order above (0..10)
 bool fused3d_encode_map(void *raw_base, const Geom &g, int esz, int variant, int field, void *map_out);
 // generic tiled tensor map (fi_fused3d.cu): nd dims, strides of dims 1..nd-1 in bytes

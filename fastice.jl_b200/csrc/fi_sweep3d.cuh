@@ -123,6 +123,15 @@ __device__ __forceinline__ T *el(unsigned slot, int li, int lj) {
 }
 #define EL(F, slot) (el<F, TX, TY, T>(slot, li, lj))
 
+// A launch chained to the one before it (programmatic stream serialization) starts when that
+// one's last blocks run: wait for its results, and let the next launch start likewise.  Set-up
+// and launch latency then overlap the sweep before (47x33x29 FP64: 11.5 -> 9.3 us an
+// iteration; 12 glaciers of 16^3-48^3 68 -> 63 us; nothing at 511^3).
+__device__ __forceinline__ void chain_launches() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename T>
 __device__ __forceinline__ T h(T x) { return T(0.5) * x; }
 
