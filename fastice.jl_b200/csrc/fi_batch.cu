@@ -18,6 +18,12 @@
 // instance's other buffer (double buffering: each sweep reads buffer s % 2 and
 // writes the other one).
 //
+// Several iterations a launch.  By default, and for up to 64 members, the sweeps between two
+// checks run on overlapping regions instead (fi_tile2d.cu): 48 members of 63^2-511^2 71.5 ->
+// 42.6 us an iteration in FP32 and 90.4 -> 53.7 in FP64.  What bounded the sweeps above was
+// the issue rate and a barrier per iteration and tile, at 40 % of the memory's.  A batch with
+// a chosen tile height, or with more members, keeps them.
+//
 // Checks.  Every ncheck sweeps a residual kernel evaluates r_P and r_V of every
 // active instance in FP64 arithmetic and folds per-instance maxima (bit patterns
 // of non-negative doubles, atomicMax: exact, order independent); a bookkeeping
@@ -582,6 +588,7 @@ struct fi_batch {
     int device = 0;
     int sms = 148;
     int variant = 0;
+    bool regions = true;  // several iterations a launch (fi_tile2d.cu); off once a tile height is chosen
     int capacity = 0;
     cudaStream_t stream = nullptr;
     void *d_inst = nullptr;               // BInst<T>[capacity]
@@ -600,14 +607,25 @@ struct fi_batch {
     BState *d_state = nullptr;
     int total_tiles = 0;
     int list_ty = -1;
+    // the regions' member table, and their tiles as the other lists
+    std::vector<unsigned char> h_reg, graph_reg;  // Tile2DTable<T>: now, and in the captured round
+    int4 *d_reg_all = nullptr, *d_reg_work = nullptr;
+    int *d_reg_first = nullptr, *d_reg_count = nullptr, *d_reg_offset = nullptr;
+    int *d_reg_ntiles = nullptr, *d_reg_full = nullptr;
+    int reg_members = 0, reg_capacity = 0, reg_tiles = 0, reg_k = 0;
+    bool reg_built = false, reg_gf = false;
     cudaGraphExec_t graph = nullptr;
-    int graph_k = -1, graph_ty = -1;
+    int graph_k = -1, graph_variant = -1;
     double graph_tol = -1;
     int graph_window = -1, graph_max = -1;
     int count() const { return (int)models.size(); }
 };
 
 namespace {
+
+// what a captured round was made of
+bool on_regions(const fi_batch *b) { return b->regions && b->count() <= kTile2DMembers; }
+int sweep_kind(const fi_batch *b) { return on_regions(b) ? -2 : b->variant; }
 
 #define FB_CHECK(expr, where)                                \
     do {                                                     \
@@ -806,6 +824,110 @@ fi_status build_tiles(fi_batch *b, int ty) {
     return FI_OK;
 }
 
+// Most iterations of one launch on regions.  Deeper launches read and write the state less
+// often and recompute more: the deepest that one wave of blocks takes, at least 4.  us per
+// iteration of 256 (one-iteration sweeps 71.5, 90.4 and 5.3): 48 members of 63^2-511^2 in FP32
+// 43.5 / 42.6 / 45.4 / 49.4 at k = 3 / 4 / 5 / 6, FP64 53.5 / 53.7 / 58.5 / 64.5; 8 members of
+// 31^2-63^2 in FP32 2.5 / 2.1 at k = 4 / 10.
+int region_depth(const fi_batch *b) {
+    auto tiles = [&](int k) {
+        long long t = 0;
+        for (const fi_model *m : b->models) {
+            int tx, ty;
+            tile2d_member_tile(m->d.grid.n[0], m->d.grid.n[1], k, &tx, &ty);
+            t += (long long)((m->d.grid.n[0] + tx) / tx) * ((m->d.grid.n[1] + ty) / ty);
+        }
+        return t;
+    };
+    for (int k = 10; k > 4; k--)
+        if (tiles(k) <= 2LL * b->sms) return k;
+    return 4;
+}
+
+// the regions' tiles (on a change of members) and table (each time, like the instance table)
+template <typename T>
+fi_status build_regions(fi_batch *b) {
+    const int n = b->count();
+    if (n == 0) return FI_OK;
+    if (!b->reg_built) {
+        b->reg_k = region_depth(b);
+        std::vector<int4> all;
+        std::vector<int> first(n), cnt(n);
+        for (int q = 0; q < n; q++) {
+            const int *c = b->models[q]->d.grid.n;
+            int tx, ty;
+            tile2d_member_tile(c[0], c[1], b->reg_k, &tx, &ty);
+            first[q] = (int)all.size();
+            for (int y = 0; y < (c[1] + ty) / ty; y++)
+                for (int x = 0; x < (c[0] + tx) / tx; x++) all.push_back(make_int4(q, x, y, 0));
+            cnt[q] = (int)all.size() - first[q];
+        }
+        const int tot = (int)all.size();
+        if (n > b->reg_members) {
+            FB_CHECK(grow(&b->d_reg_first, n), "region arrays");
+            FB_CHECK(grow(&b->d_reg_count, n), "region arrays");
+            FB_CHECK(grow(&b->d_reg_offset, n), "region arrays");
+            FB_CHECK(grow(&b->d_reg_ntiles, 1), "region arrays");
+            FB_CHECK(grow(&b->d_reg_full, 1), "region arrays");
+            b->reg_members = n;
+        }
+        if (tot > b->reg_capacity) {
+            FB_CHECK(grow(&b->d_reg_all, tot), "region list");
+            FB_CHECK(grow(&b->d_reg_work, tot), "region list");
+            b->reg_capacity = tot;
+        }
+        FB_CHECK(cudaMemcpy(b->d_reg_all, all.data(), sizeof(int4) * tot, cudaMemcpyHostToDevice), "region list");
+        FB_CHECK(cudaMemcpy(b->d_reg_work, all.data(), sizeof(int4) * tot, cudaMemcpyHostToDevice), "region list");
+        FB_CHECK(cudaMemcpy(b->d_reg_first, first.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "region offsets");
+        FB_CHECK(cudaMemcpy(b->d_reg_count, cnt.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "region counts");
+        FB_CHECK(cudaMemcpy(b->d_reg_full, &tot, sizeof(int), cudaMemcpyHostToDevice), "region total");
+        FB_CHECK(cudaMemcpy(b->d_reg_ntiles, &tot, sizeof(int), cudaMemcpyHostToDevice), "region total");
+        b->reg_tiles = tot;
+        b->reg_built = true;
+        if (b->graph) cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    b->h_reg.assign(sizeof(Tile2DTable<T>), 0);
+    Tile2DTable<T> *tab = reinterpret_cast<Tile2DTable<T> *>(b->h_reg.data());
+    bool gf = false;
+    for (int q = 0; q < n; q++) {
+        const BInst<T> &v = reinterpret_cast<const BInst<T> *>(b->h_inst.data())[q];
+        Tile2DMember<T> &u = tab->m[q];
+        u.n[0] = v.n0, u.n[1] = v.n1, u.pitch = (int)v.pitch, u.forced = v.pforce;
+        tile2d_member_tile(v.n0, v.n1, b->reg_k, &u.tx, &u.ty);
+        std::memcpy(u.bc_kind, v.bc_kind, sizeof(u.bc_kind));
+        std::memcpy(u.bc_val, v.bc_val, sizeof(u.bc_val));
+        u.inv_dx[0] = v.idx, u.inv_dx[1] = v.idy, u.dt_P = v.dtP;
+        u.dt_tau[0] = v.dxx, u.dt_tau[1] = v.dyy, u.dt_tau[2] = v.dxy;
+        u.dt_V[0] = v.dVx, u.dt_V[1] = v.dVy;
+        for (int c = 0; c < 2; c++) {
+            u.g_kind[c] = v.gkind[c], u.g_val[c] = v.gval[c];
+            T *f[6] = {v.P[c], v.txx[c], v.tyy[c], v.txy[c], v.Vx[c], v.Vy[c]};
+            std::memcpy(u.f[c], f, sizeof(f));
+            gf = gf || v.gkind[c] == FI_G_FIELD;
+        }
+        u.eta = v.eta, u.gx = v.gx, u.gy = v.gy, u.fP = v.fP;
+    }
+    b->reg_gf = gf;
+    return FI_OK;
+}
+
+// k iterations on regions: launches of at most reg_k, their number of the parity of k, so
+// that an even k leaves the state in its buffers
+template <typename T>
+cudaError_t launch_regions(fi_batch *b, const int4 *list, const int *nt, int k) {
+    int L = (k + b->reg_k - 1) / b->reg_k;
+    L += (L ^ k) & 1;
+    cudaError_t e = cudaSuccess;
+    for (int l = 0, left = k; l < L && e == cudaSuccess; l++) {
+        const int step = (left + L - l - 1) / (L - l);
+        left -= step;
+        e = launch_tile2d_batched<T>(*reinterpret_cast<const Tile2DTable<T> *>(b->h_reg.data()), list, nt, b->reg_tiles, l & 1, step, b->reg_gf, l > 0,
+                                     b->stream);
+    }
+    return e;
+}
+
 template <typename T, int TY>
 cudaError_t launch_sweep_t(fi_batch *b, const int4 *list, const int *nt, int src) {
     const int grid = b->sms * sweep_blocks_per_sm<T, TY>();
@@ -823,6 +945,20 @@ cudaError_t launch_sweep_ty(fi_batch *b, const int4 *list, const int *nt, int sr
 }
 cudaError_t launch_sweep(fi_batch *b, const int4 *list, const int *nt, int src) {
     return b->f64 ? launch_sweep_ty<double>(b, list, nt, src) : launch_sweep_ty<float>(b, list, nt, src);
+}
+
+
+// k sweeps of every member (all) or of the active ones
+cudaError_t launch_sweeps(fi_batch *b, bool all, int k) {
+    if (on_regions(b)) {
+        const int4 *list = all ? b->d_reg_all : b->d_reg_work;
+        const int *nt = all ? b->d_reg_full : b->d_reg_ntiles;
+        return b->f64 ? launch_regions<double>(b, list, nt, k) : launch_regions<float>(b, list, nt, k);
+    }
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < k && e == cudaSuccess; s++)
+        e = launch_sweep(b, all ? b->d_all : b->d_work, all ? b->d_full_ntiles : b->d_ntiles, s & 1);
+    return e;
 }
 
 template <typename T, int TY>
@@ -846,14 +982,18 @@ cudaError_t enqueue_compaction(fi_batch *b) {
     if (e != cudaSuccess) return e;
     batch_fill<<<std::max(1, std::min((b->total_tiles + 255) / 256, b->sms * 8)), 256, 0, b->stream>>>(
         b->total_tiles, b->d_all, b->d_first, b->d_offset, b->d_state, b->d_work);
+    if ((e = cudaGetLastError()) != cudaSuccess || !on_regions(b)) return e;
+    batch_scan<<<1, 1024, 0, b->stream>>>(b->count(), b->d_reg_count, b->d_state, b->d_reg_offset, b->d_reg_ntiles, b->d_nactive);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    batch_fill<<<std::max(1, std::min((b->reg_tiles + 255) / 256, b->sms * 8)), 256, 0, b->stream>>>(
+        b->reg_tiles, b->d_reg_all, b->d_reg_first, b->d_reg_offset, b->d_state, b->d_reg_work);
     return cudaGetLastError();
 }
 
 // one check-to-check step: k sweeps, the check, bookkeeping, compaction
 cudaError_t enqueue_round(fi_batch *b, int k, double tol, int window, int max_iter) {
     cudaError_t e;
-    for (int s = 0; s < k; s++)
-        if ((e = launch_sweep(b, b->d_work, b->d_ntiles, s & 1)) != cudaSuccess) return e;
+    if ((e = launch_sweeps(b, false, k)) != cudaSuccess) return e;
     if ((e = launch_check(b, b->d_work, b->d_ntiles)) != cudaSuccess) return e;
     batch_update<<<(b->count() + 255) / 256, 256, 0, b->stream>>>(b->count(), b->d_h, b->d_slots, b->d_state, k, tol,
                                                                    window, max_iter);
@@ -870,11 +1010,13 @@ fi_status prepare(fi_batch *b) {
         if ((st = model_ensure_second_state(m)) != FI_OK) return st;
     }
     if (b->dirty) {
+        b->reg_built = false;
         if ((st = pull_state(b)) != FI_OK) return st;
         if ((st = ensure_capacity(b)) != FI_OK) return st;
     }
     if ((st = upload_table(b)) != FI_OK) return st;
     if ((st = build_tiles(b, kBatchTY[b->variant])) != FI_OK) return st;
+    if (on_regions(b) && (st = b->f64 ? build_regions<double>(b) : build_regions<float>(b)) != FI_OK) return st;
     if (!b->state_on_device) {
         if (b->count() > 0)
             FB_CHECK(cudaMemcpy(b->d_state, b->h_state.data(), sizeof(BState) * b->count(), cudaMemcpyHostToDevice),
@@ -889,7 +1031,9 @@ void free_batch(fi_batch *b) {
     if (!b) return;
     if (b->graph) cudaGraphExecDestroy(b->graph);
     void *ptrs[] = {b->d_inst, b->d_all, b->d_work, b->d_first, b->d_count, b->d_offset, b->d_ntiles,
-                    b->d_nactive, b->d_full_ntiles, b->d_h, b->d_slots, b->d_state, b->d_maps, b->d_err};
+                    b->d_nactive, b->d_full_ntiles, b->d_h, b->d_slots, b->d_state, b->d_maps, b->d_err,
+                    b->d_reg_all, b->d_reg_work, b->d_reg_first, b->d_reg_count, b->d_reg_offset, b->d_reg_ntiles,
+                    b->d_reg_full};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (b->h_nactive) cudaFreeHost(b->h_nactive);
@@ -926,7 +1070,7 @@ fi_status run_rounds(fi_batch *b, const fi_batch_opts *o, int max_rounds, fi_bat
     const int window = o->window > 0 ? o->window : 0;
     const bool use_graph = o->use_graph != 0;
     if (use_graph && *b->h_nactive > 0 &&
-        (!b->graph || b->graph_k != o->ncheck || b->graph_ty != kBatchTY[b->variant] || b->graph_tol != o->tol ||
+        (!b->graph || b->graph_k != o->ncheck || (on_regions(b) && b->graph_reg != b->h_reg) || b->graph_variant != sweep_kind(b) || b->graph_tol != o->tol ||
          b->graph_window != window || b->graph_max != o->max_iter)) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -940,7 +1084,8 @@ fi_status run_rounds(fi_batch *b, const fi_batch_opts *o, int max_rounds, fi_bat
         cudaGraphDestroy(g);
         if (ie != cudaSuccess) return cuda_fail(ie, "graph instantiate");
         b->graph_k = o->ncheck;
-        b->graph_ty = kBatchTY[b->variant];
+        b->graph_variant = sweep_kind(b);
+        b->graph_reg = b->h_reg;
         b->graph_tol = o->tol;
         b->graph_window = window;
         b->graph_max = o->max_iter;
@@ -1067,7 +1212,7 @@ fi_status fi_batch_advance(fi_batch *b, int32_t niter) {
     if (!b || niter < 0) return set_error("bad argument"), FI_ERR_ARG;
     fi_status st = prepare(b);
     if (st != FI_OK) return st;
-    for (int s = 0; s < niter; s++) FB_CHECK(launch_sweep(b, b->d_all, b->d_full_ntiles, s & 1), "batch sweep");
+    FB_CHECK(launch_sweeps(b, true, niter), "batch sweep");
     FB_CHECK(cudaStreamSynchronize(b->stream), "batch sync");
     finish_sweeps(b, std::vector<int>(b->count(), niter));
     return check_batch_err(b);
@@ -1076,6 +1221,7 @@ fi_status fi_batch_advance(fi_batch *b, int32_t niter) {
 fi_status fi_batch_set_variant(fi_batch *b, int32_t v) {
     if (!b || v < 0 || v >= kBatchVariants) return set_error("bad argument"), FI_ERR_ARG;
     b->variant = v;
+    b->regions = false;
     return FI_OK;
 }
 
@@ -1088,11 +1234,14 @@ fi_status fi_batch_autotune(fi_batch *b, int32_t iters, int32_t *best, double *m
     double best_ms = 1e300;
     int best_v = 0;
     fi_status st = FI_OK;
+    // the tile heights of one-iteration sweeps (and of the checks); a batch on regions stays there
+    const bool regions = b->regions;
+    b->regions = false;
     for (int v = 0; v < kBatchVariants && st == FI_OK; v++) {
         b->variant = v;
         if ((st = fi_batch_advance(b, 2)) != FI_OK) break;  // warm-up (and the variant's tile list)
         cudaEventRecord(e0, b->stream);
-        for (int s = 0; s < iters; s++) launch_sweep(b, b->d_all, b->d_full_ntiles, s & 1);
+        launch_sweeps(b, true, iters);
         cudaEventRecord(e1, b->stream);
         cudaError_t e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) {
@@ -1111,6 +1260,7 @@ fi_status fi_batch_autotune(fi_batch *b, int32_t iters, int32_t *best, double *m
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    b->regions = regions;
     if (st != FI_OK) return st;
     if ((st = check_batch_err(b)) != FI_OK) return st;
     b->variant = best_v;
@@ -1168,6 +1318,7 @@ fi_status fi_batch_solve_mixed(fi_batch *b, const fi_batch_opts *o, double inner
         ~Guard() { fi_batch_destroy(p); }
     } guard{sb};
     sb->variant = b->variant;
+    sb->regions = b->regions;
     std::vector<int> sweeps(n, 0), status(n, FI_ITEM_ACTIVE), stale(n, 0);
     std::vector<double> best(n, 1e300), meas(n, 0.0);
     std::vector<fi_batch_item> it(n);

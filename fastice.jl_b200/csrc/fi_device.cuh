@@ -123,8 +123,9 @@ __device__ __forceinline__ T sum_r(T a, T i, T b, T j) { return fma_r(a, i, mul_
 template <typename T>
 __device__ __forceinline__ T relax_r(T o, T e, T r, T dt) { return fma_r(-fma_r(-e, r, o), dt, o); }
 // The divergence of the differences s0, s1 (, s2) over the spacings 1/i and the deviators of
-// their rates (ND 2: d[2] is not set)
-template <int ND, typename T>
+// their rates (ND 2: d[2] is not set).  SUMS: of rounded rates, as the FP32 kernels and the
+// batched 2D sweeps come out; else as the FP64 kernels.
+template <int ND, bool SUMS, typename T>
 __device__ __forceinline__ T rates_r(const T (&s)[3], const T *i, T (&d)[3]) {
     const T e0 = mul_r(s[0], i[0]), e1 = mul_r(s[1], i[1]), e2 = ND == 3 ? mul_r(s[2], i[2]) : T(0);
 #ifdef FI_EXACT_ORDER
@@ -132,7 +133,7 @@ __device__ __forceinline__ T rates_r(const T (&s)[3], const T *i, T (&d)[3]) {
     d[0] = e0 - t, d[1] = e1 - t, d[2] = e2 - t;
 #else
     T v;
-    if (sizeof(T) == 8) {
+    if (!SUMS) {
         v = fma_r(s[0], i[0], e1);
         if (ND == 3) v = fma_r(s[2], i[2], v);
         const T t = mul_r(v, T(1.0 / 3.0));

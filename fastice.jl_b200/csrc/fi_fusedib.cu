@@ -94,7 +94,7 @@ __device__ __forceinline__ Centre<T> centre_masked(const Ctx<T, TX, TY> &c, cons
     const T e2 = T(2.0) * *EL(M_ET, c.V0);
     const T s[3] = {diff_r(w.nxr, vx[1], w.nx, vx[0]), diff_r(w.nyt, vy[BV], w.ny, vy[0]), diff_r(w.nzu, vzp[0], w.nz, vz[0])};
     T d[3];
-    const T divV = rates_r<3>(s, q.inv_dx, d);
+    const T divV = rates_r<3, sizeof(T) == 4>(s, q.inv_dx, d);
     const T dv = p.p_forcing && on ? divV + __ldg(in.fP + I) : divV;
     auto pick = [&](T o, T r, int k) { return on ? relax_r(o, e2, r, q.dt_tau[k]) : o; };
     Centre<T> r;

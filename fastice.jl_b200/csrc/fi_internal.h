@@ -234,6 +234,29 @@ template <typename T>
 cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, T *eta_prev, int shape,
                           int k, bool write_prev, cudaStream_t s);
 
+// The same for the members of a batch: work item = (member, tile x, tile y).  What the kernel
+// needs of a member; f[src] is read, f[src ^ 1] written (P, τxx, τyy, τxy, V.x, V.y); η fixed.
+template <typename T>
+struct Tile2DMember {
+    int n[2], tx, ty;  // cells; the member's tile (tile2d_member_tile)
+    int pitch, forced, bc_kind[2][2], g_kind[2];
+    T inv_dx[2], dt_P, dt_tau[3], dt_V[2], g_val[2], bc_val[2][2][2];
+    const T *eta, *gx, *gy, *fP;
+    T *f[2][6];
+};
+// a launch's members: kernel arguments, so that an iteration finds them in the constant bank
+constexpr int kTile2DMembers = 64;
+template <typename T>
+struct Tile2DTable {
+    Tile2DMember<T> m[kTile2DMembers];
+};
+// tile sides of an n0 x n1 grid for launches of at most k iterations
+void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty);
+// gf: some member's body force is a field; chained: right after another of these launches
+template <typename T>
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
+                                  int k, bool gf, bool chained, cudaStream_t s);
+
 // ---- mixed-precision solve helpers (fi_mixed.cu) ----
 template <typename S, typename D>
 cudaError_t launch_convert(const S *src, D *dst, long long n, double scale, cudaStream_t s);

@@ -81,7 +81,7 @@ struct Strip {
 // The k iterations of a region.  EDGE: it touches a side that is not periodic.  Every point
 // computes; where no such value exists the result is not stored, and what the strip keeps
 // of it is replaced by the ghost that another thread has put there.
-template <bool EDGE, bool GF, typename T, int RX, int RY, int PY>
+template <bool EDGE, bool GF, bool BATCH, typename T, int RX, int RY, int PY>
 __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, const Ptrs<T> &in, Strip<T, PY> &v, T *sP, int a0,
                                         int k) {
     using R = Region<T, RX, RY, PY>;
@@ -104,7 +104,7 @@ __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, co
             etd[r] = ed;
             const T s[3] = {sVx[a + 1] - v.vx[r], vyu - v.vy[r], T(0)};
             T d[3];
-            const T divV = rates_r<2>(s, q.inv_dx, d);
+            const T divV = rates_r<2, BATCH || sizeof(T) == 4>(s, q.inv_dx, d);
             const T exy = h(sum_r(v.vy[r] - sVy[a - 1], idx, v.vx[r] - vxd, idy));
             const T dv = forced ? divV + __ldg(in.fP + v.at[r]) : divV;
             const T nP = fma_r(-mul_r(dv, v.et[r]), q.dt_P, v.P[r]);
@@ -223,18 +223,20 @@ __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, co
     }
 }
 
-template <typename T, int RX, int RY, int PY, int MINB, bool GF>
-__global__ void __launch_bounds__(RX *RY / PY, MINB)
-    tile2d_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, T *eta_prev, TileArgs ta) {
+// one region, the one around tile (bx, by)
+template <typename T, int RX, int RY, int PY, bool GF, bool BATCH>
+__device__ __forceinline__ void run_region(const Geom &g, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
+                                           const Ptrs<T> &out, T *eta_prev, const TileArgs &ta, int bx, int by,
+                                           unsigned char *t2_smem) {
     using R = Region<T, RX, RY, PY>;
     constexpr int PW = R::PW;
-    extern __shared__ __align__(16) unsigned char t2_smem[];
     T *sP = reinterpret_cast<T *>(t2_smem), *sXX = sP + R::PLANE, *sYY = sXX + R::PLANE, *sXY = sYY + R::PLANE;
     T *sVx = sXY + R::PLANE, *sVy = sVx + R::PLANE, *sE = sVy + R::PLANE;
     const int w = threadIdx.x / 32, x = threadIdx.x % 32 + 32 * (w % (RX / 32)), y0 = (w / (RX / 32)) * PY;
     const int n0 = g.n[0], n1 = g.n[1];
-    const bool px = p.bc_kind[0][0] == FI_BC_PERIODIC, py = p.bc_kind[1][0] == FI_BC_PERIODIC;
-    const int i0 = 1 + (int)blockIdx.x * ta.tx - ta.k, j0 = 1 + (int)blockIdx.y * ta.ty - ta.k;
+    // (a batch has no periodic members)
+    const bool px = !BATCH && p.bc_kind[0][0] == FI_BC_PERIODIC, py = !BATCH && p.bc_kind[1][0] == FI_BC_PERIODIC;
+    const int i0 = 1 + bx * ta.tx - ta.k, j0 = 1 + by * ta.ty - ta.k;
     const int gi = i0 + x;
     const int a0 = (y0 + 1) * PW + x + 1;
     const bool edge = (!px && (i0 <= 1 || i0 + RX > n0)) || (!py && (j0 <= 1 || j0 + RY > n1));
@@ -307,8 +309,8 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
         sE[a] = v.et[r];
     }
     __syncthreads();
-    if (edge) iterate<true, GF, T, RX, RY, PY>(p, q, in, v, sP, a0, ta.k);
-    else iterate<false, GF, T, RX, RY, PY>(p, q, in, v, sP, a0, ta.k);
+    if (edge) iterate<true, GF, BATCH, T, RX, RY, PY>(p, q, in, v, sP, a0, ta.k);
+    else iterate<false, GF, BATCH, T, RX, RY, PY>(p, q, in, v, sP, a0, ta.k);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- the inner tile (with the ghosts beside it) to the other buffer ----
@@ -351,6 +353,64 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
 }
 
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
+__global__ void __launch_bounds__(RX *RY / PY, MINB)
+    tile2d_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, T *eta_prev, TileArgs ta) {
+    extern __shared__ __align__(16) unsigned char t2_smem[];
+    run_region<T, RX, RY, PY, GF, false>(g, p, q, in, out, eta_prev, ta, (int)blockIdx.x, (int)blockIdx.y, t2_smem);
+}
+
+// The regions of several models, a block each; blocks past the end of the work list leave.
+// The list does not change while chained launches run.  The members come as kernel arguments:
+// copied from a device table into shared memory they cost the iterations' loads and registers
+// (48 members of 63^2-511^2, FP32: 60.6 us an iteration; a persistent grid that copies the
+// next member ahead 67.4), as uniform operands from the constant bank 42.6.
+template <typename T, int RX, int RY, int PY, int MINB, bool GF>
+__global__ void __launch_bounds__(RX *RY / PY, MINB)
+    tile2d_batched(const __grid_constant__ Tile2DTable<T> members, const int4 *__restrict__ tiles,
+                   const int *__restrict__ ntiles, int src, int k) {
+    extern __shared__ __align__(16) unsigned char t2_smem[];
+    if ((int)blockIdx.x >= *ntiles) return;
+    const int4 d = tiles[blockIdx.x];
+    // (a reduction's result is known to be the same in all lanes: the member's values are
+    // read as uniform operands)
+    const Tile2DMember<T> &c = members.m[__reduce_max_sync(0xffffffffu, (unsigned)d.x)];
+    Geom g{};
+    KParams p{};
+    TConst<T> q{};
+    Ptrs<T> in{}, out{};
+    p.freeze_eta = 1;
+    p.p_forcing = c.forced;
+    q.dt_P = c.dt_P;
+    q.dt_tau[0] = c.dt_tau[0], q.dt_tau[1] = c.dt_tau[1], q.dt_tau[3] = c.dt_tau[2];
+    g.pitch = c.pitch;
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        g.n[a] = c.n[a];
+        p.g_kind[a] = c.g_kind[a];
+        q.inv_dx[a] = c.inv_dx[a], q.dt_V[a] = c.dt_V[a], q.g_val[a] = c.g_val[a];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            p.bc_kind[a][e] = c.bc_kind[a][e];
+            q.bc_val[a][e][0] = c.bc_val[a][e][0], q.bc_val[a][e][1] = c.bc_val[a][e][1];
+        }
+    }
+    in.P = c.f[src][0], in.txx = c.f[src][1], in.tyy = c.f[src][2], in.txy = c.f[src][3], in.Vx = c.f[src][4], in.Vy = c.f[src][5];
+    in.eta = const_cast<T *>(c.eta), in.gx = c.gx, in.gy = c.gy, in.fP = const_cast<T *>(c.fP);
+    const int dst = src ^ 1;
+    out.P = c.f[dst][0], out.txx = c.f[dst][1], out.tyy = c.f[dst][2], out.txy = c.f[dst][3], out.Vx = c.f[dst][4],
+    out.Vy = c.f[dst][5];
+    const TileArgs ta{k, c.tx, c.ty, 0};
+    run_region<T, RX, RY, PY, GF, true>(g, p, q, in, out, nullptr, ta, d.y, d.z, t2_smem);
+}
+
+// No tile starts at the last node of a bounded dimension: the ghosts there follow from the
+// cell before it, which would lie outside what the region gets right.
+int inner_tile(int t, int n, bool per) {
+    while (!per && t > 2 && n % t == 0) t--;
+    return t;
+}
+
+template <typename T, int RX, int RY, int PY, int MINB, bool GF>
 cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, T *eta_prev, int k,
                           bool write_prev, cudaStream_t s) {
     using R = Region<T, RX, RY, PY>;
@@ -365,13 +425,7 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
     }
     const bool px = p.bc_kind[0][0] == FI_BC_PERIODIC, py = p.bc_kind[1][0] == FI_BC_PERIODIC;
     const int ex = px ? g.n[0] : g.n[0] + 1, ey = py ? g.n[1] : g.n[1] + 1;
-    // no tile starts at the last node of a bounded dimension: the ghosts there follow from the
-    // cell before it, which would lie outside what the region gets right
-    auto inner = [](int t, int n, bool per) {
-        while (!per && t > 2 && n % t == 0) t--;
-        return t;
-    };
-    const TileArgs ta{k, inner(RX - 2 * k, g.n[0], px), inner(RY - 2 * k, g.n[1], py), write_prev ? 1 : 0};
+    const TileArgs ta{k, inner_tile(RX - 2 * k, g.n[0], px), inner_tile(RY - 2 * k, g.n[1], py), write_prev ? 1 : 0};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((ex + ta.tx - 1) / ta.tx, (ey + ta.ty - 1) / ta.ty);
     cfg.blockDim = dim3(R::NT);
@@ -384,6 +438,32 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, g, p, make_tconst<T>(p), in, out, eta_prev, ta);
+}
+
+template <typename T, bool GF>
+cudaError_t launch_batched_regions(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
+                                   int k, bool chained, cudaStream_t s) {
+    using R = Region<T, 32, 32, 2>;
+    auto *kern = tile2d_batched<T, 32, 32, 2, 2, GF>;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static bool attr_set[64] = {};
+    if (dev < 64 && !attr_set[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::SMEM);
+        if (e != cudaSuccess) return e;
+        attr_set[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(max_tiles);
+    cfg.blockDim = dim3(R::NT);
+    cfg.dynamicSmemBytes = R::SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, members, tiles, ntiles, src, k);
 }
 
 }  // namespace
@@ -430,6 +510,23 @@ cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, co
               : launch_shape<T, false>(g, p, in, out, eta_prev, shape, k, write_prev, s);
 }
 
+void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty) {
+    *tx = inner_tile(32 - 2 * k, n0, false);
+    *ty = inner_tile(32 - 2 * k, n1, false);
+}
+
+template <typename T>
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
+                                  int k, bool gf, bool chained, cudaStream_t s) {
+    if (max_tiles <= 0) return cudaSuccess;
+    return gf ? launch_batched_regions<T, true>(members, tiles, ntiles, max_tiles, src, k, chained, s)
+              : launch_batched_regions<T, false>(members, tiles, ntiles, max_tiles, src, k, chained, s);
+}
+
+template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, const int4 *, const int *, int, int, int, bool,
+                                                   bool, cudaStream_t);
+template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, const int4 *, const int *, int, int, int, bool,
+                                                  bool, cudaStream_t);
 template cudaError_t launch_tile2d<double>(const Geom &, const KParams &, const Ptrs<double> &, const Ptrs<double> &, double *,
                                            int, int, bool, cudaStream_t);
 template cudaError_t launch_tile2d<float>(const Geom &, const KParams &, const Ptrs<float> &, const Ptrs<float> &, float *, int,
