@@ -888,6 +888,7 @@ fi_status fi_model_destroy(fi_model *m) {
     if (m->d_blist) cudaFree(m->d_blist);
     if (m->d_bcount) cudaFree(m->d_bcount);
     if (m->d_jobs) cudaFree(m->d_jobs);
+    host_stage_release(&m->host_stage);
     for (cudaGraphExec_t &g : m->pair_graph)
         if (g) cudaGraphExecDestroy(g);
     field_free(m->fP, m->esz);
@@ -936,8 +937,7 @@ fi_status fi_model_get_field(fi_model *m, int32_t field, void *host, size_t nbyt
     if (is_residual(field) && !m->base[field]) return set_error("residuals not computed yet"), FI_ERR_STATE;
     FI_CHECK_CUDA(cudaSetDevice(m->d.device), "cudaSetDevice");
     cudaMemcpy3DParms p = copy_params(m, field, m->cur(field), host, false);
-    FI_CHECK_CUDA(cudaMemcpy3DAsync(&p, m->stream), "get_field copy");
-    FI_CHECK_CUDA(cudaStreamSynchronize(m->stream), "get_field sync");
+    FI_CHECK_CUDA(host_download(p, m->d.device, m->stream, &m->host_stage), "get_field copy");
     return FI_OK;
 }
 

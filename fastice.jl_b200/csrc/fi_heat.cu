@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <string>
 
+#include "fi_hostcopy.h"
 #include "fi_internal.h"
 
 #define FI_CHECK_CUDA(expr, where)                          \
@@ -34,6 +35,7 @@ struct fi_heat {
     void *T[2] = {}, *q[3][2] = {}, *To = nullptr;
     int cur = 0;  // buffer holding the current T and q
     cudaStream_t stream = nullptr;
+    fi::HostStage stage;  // of get_field into pageable memory
 };
 
 namespace fi {
@@ -302,6 +304,7 @@ fi_status fi_heat_destroy(fi_heat *h) {
     if (!h) return FI_OK;
     cudaSetDevice(h->d.device);
     cudaStreamSynchronize(h->stream);
+    host_stage_release(&h->stage);
     heat_free(h);
     return FI_OK;
 }
@@ -333,8 +336,7 @@ fi_status fi_heat_get_field(fi_heat *h, int32_t field, void *host, size_t nbytes
     if (!host || nbytes != cnt * h->esz) return set_error("byte count does not match the field's interior"), FI_ERR_ARG;
     FI_CHECK_CUDA(cudaSetDevice(h->d.device), "cudaSetDevice");
     cudaMemcpy3DParms p = heat_copy(h, field, heat_ptr(h, field, h->cur), host, false);
-    FI_CHECK_CUDA(cudaMemcpy3DAsync(&p, h->stream), "heat get_field");
-    FI_CHECK_CUDA(cudaStreamSynchronize(h->stream), "heat get_field");
+    FI_CHECK_CUDA(host_download(p, h->d.device, h->stream, &h->stage), "heat get_field");
     return FI_OK;
 }
 

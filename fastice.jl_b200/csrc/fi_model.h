@@ -4,6 +4,7 @@
 #pragma once
 
 #include "fi_fusedib.h"
+#include "fi_hostcopy.h"
 #include "fi_internal.h"
 
 namespace fi {
@@ -70,6 +71,7 @@ struct fi_model {
     int4 *d_jobs = nullptr;
     int n_jobs = 0;
     void *fP = nullptr;    // pressure forcing (defect-correction shadow models only)
+    fi::HostStage host_stage;  // of get_field into pageable memory
     void *d_stage = nullptr;  // staging buffer of set_field (contiguous rows of host data)
     size_t stage_bytes = 0;
     fi_model *shadow = nullptr;  // FP32 model of the mixed-precision solve (created on first use)
