@@ -18,11 +18,11 @@
 // instance's other buffer (double buffering: each sweep reads buffer s % 2 and
 // writes the other one).
 //
-// Several iterations a launch.  By default, and for up to 64 members, the sweeps between two
-// checks run on overlapping regions instead (fi_tile2d.cu): 48 members of 63^2-511^2 71.5 ->
-// 42.6 us an iteration in FP32 and 90.4 -> 53.7 in FP64.  What bounded the sweeps above was
-// the issue rate and a barrier per iteration and tile, at 40 % of the memory's.  A batch with
-// a chosen tile height, or with more members, keeps them.
+// Several iterations a launch.  By default the sweeps between two checks run on overlapping
+// regions instead (fi_tile2d.cu), a launch per 64 members (their parameters are kernel
+// arguments): 48 members of 63^2-511^2 71.5 -> 42.6 us an iteration in FP32 and 90.4 -> 53.7
+// in FP64, 256 members 448 -> 279 and 632 -> 351.  What bounded the sweeps above was the issue rate and a barrier per
+// iteration and tile, at 40 % of the memory's.  A batch with a chosen tile height keeps them.
 //
 // Checks.  Every ncheck sweeps a residual kernel evaluates r_P and r_V of every
 // active instance in FP64 arithmetic and folds per-instance maxima (bit patterns
@@ -608,7 +608,8 @@ struct fi_batch {
     int total_tiles = 0;
     int list_ty = -1;
     // the regions' member table, and their tiles as the other lists
-    std::vector<unsigned char> h_reg, graph_reg;  // Tile2DTable<T>: now, and in the captured round
+    std::vector<unsigned char> h_reg, graph_reg;  // Tile2DTable<T> per group of members: now, and in the captured round
+    std::vector<int> reg_max;                     // tiles of each group
     int4 *d_reg_all = nullptr, *d_reg_work = nullptr;
     int *d_reg_first = nullptr, *d_reg_count = nullptr, *d_reg_offset = nullptr;
     int *d_reg_ntiles = nullptr, *d_reg_full = nullptr;
@@ -624,8 +625,7 @@ struct fi_batch {
 namespace {
 
 // what a captured round was made of
-bool on_regions(const fi_batch *b) { return b->regions && b->count() <= kTile2DMembers; }
-int sweep_kind(const fi_batch *b) { return on_regions(b) ? -2 : b->variant; }
+int sweep_kind(const fi_batch *b) { return b->regions ? -2 : b->variant; }
 
 #define FB_CHECK(expr, where)                                \
     do {                                                     \
@@ -883,16 +883,18 @@ fi_status build_regions(fi_batch *b) {
         FB_CHECK(cudaMemcpy(b->d_reg_full, &tot, sizeof(int), cudaMemcpyHostToDevice), "region total");
         FB_CHECK(cudaMemcpy(b->d_reg_ntiles, &tot, sizeof(int), cudaMemcpyHostToDevice), "region total");
         b->reg_tiles = tot;
+        b->reg_max.assign((n + kTile2DMembers - 1) / kTile2DMembers, 0);
+        for (int q = 0; q < n; q++) b->reg_max[q / kTile2DMembers] += cnt[q];
         b->reg_built = true;
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    b->h_reg.assign(sizeof(Tile2DTable<T>), 0);
+    b->h_reg.assign(sizeof(Tile2DTable<T>) * b->reg_max.size(), 0);
     Tile2DTable<T> *tab = reinterpret_cast<Tile2DTable<T> *>(b->h_reg.data());
     bool gf = false;
     for (int q = 0; q < n; q++) {
         const BInst<T> &v = reinterpret_cast<const BInst<T> *>(b->h_inst.data())[q];
-        Tile2DMember<T> &u = tab->m[q];
+        Tile2DMember<T> &u = tab[q / kTile2DMembers].m[q % kTile2DMembers];
         u.n[0] = v.n0, u.n[1] = v.n1, u.pitch = (int)v.pitch, u.forced = v.pforce;
         tile2d_member_tile(v.n0, v.n1, b->reg_k, &u.tx, &u.ty);
         std::memcpy(u.bc_kind, v.bc_kind, sizeof(u.bc_kind));
@@ -915,15 +917,20 @@ fi_status build_regions(fi_batch *b) {
 // k iterations on regions: launches of at most reg_k, their number of the parity of k, so
 // that an even k leaves the state in its buffers
 template <typename T>
-cudaError_t launch_regions(fi_batch *b, const int4 *list, const int *nt, int k) {
+cudaError_t launch_regions(fi_batch *b, bool all, int k) {
+    const int4 *list = all ? b->d_reg_all : b->d_reg_work;
+    const int *start = all ? b->d_reg_first : b->d_reg_offset, *nt = all ? b->d_reg_full : b->d_reg_ntiles;
+    const Tile2DTable<T> *tab = reinterpret_cast<const Tile2DTable<T> *>(b->h_reg.data());
+    const int groups = (int)b->reg_max.size();
     int L = (k + b->reg_k - 1) / b->reg_k;
     L += (L ^ k) & 1;
     cudaError_t e = cudaSuccess;
     for (int l = 0, left = k; l < L && e == cudaSuccess; l++) {
         const int step = (left + L - l - 1) / (L - l);
         left -= step;
-        e = launch_tile2d_batched<T>(*reinterpret_cast<const Tile2DTable<T> *>(b->h_reg.data()), list, nt, b->reg_tiles, l & 1, step, b->reg_gf, l > 0,
-                                     b->stream);
+        for (int c = 0; c < groups && e == cudaSuccess; c++)
+            e = launch_tile2d_batched<T>(tab[c], c * kTile2DMembers, c == groups - 1, list, start, nt, b->reg_max[c], l & 1, step,
+                                         b->reg_gf, l + c > 0, b->stream);
     }
     return e;
 }
@@ -950,11 +957,8 @@ cudaError_t launch_sweep(fi_batch *b, const int4 *list, const int *nt, int src) 
 
 // k sweeps of every member (all) or of the active ones
 cudaError_t launch_sweeps(fi_batch *b, bool all, int k) {
-    if (on_regions(b)) {
-        const int4 *list = all ? b->d_reg_all : b->d_reg_work;
-        const int *nt = all ? b->d_reg_full : b->d_reg_ntiles;
-        return b->f64 ? launch_regions<double>(b, list, nt, k) : launch_regions<float>(b, list, nt, k);
-    }
+    if (b->count() == 0) return cudaSuccess;  // (the lists are those of the last members)
+    if (b->regions) return b->f64 ? launch_regions<double>(b, all, k) : launch_regions<float>(b, all, k);
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < k && e == cudaSuccess; s++)
         e = launch_sweep(b, all ? b->d_all : b->d_work, all ? b->d_full_ntiles : b->d_ntiles, s & 1);
@@ -982,7 +986,7 @@ cudaError_t enqueue_compaction(fi_batch *b) {
     if (e != cudaSuccess) return e;
     batch_fill<<<std::max(1, std::min((b->total_tiles + 255) / 256, b->sms * 8)), 256, 0, b->stream>>>(
         b->total_tiles, b->d_all, b->d_first, b->d_offset, b->d_state, b->d_work);
-    if ((e = cudaGetLastError()) != cudaSuccess || !on_regions(b)) return e;
+    if ((e = cudaGetLastError()) != cudaSuccess || !b->regions || b->count() == 0) return e;
     batch_scan<<<1, 1024, 0, b->stream>>>(b->count(), b->d_reg_count, b->d_state, b->d_reg_offset, b->d_reg_ntiles, b->d_nactive);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     batch_fill<<<std::max(1, std::min((b->reg_tiles + 255) / 256, b->sms * 8)), 256, 0, b->stream>>>(
@@ -1016,7 +1020,7 @@ fi_status prepare(fi_batch *b) {
     }
     if ((st = upload_table(b)) != FI_OK) return st;
     if ((st = build_tiles(b, kBatchTY[b->variant])) != FI_OK) return st;
-    if (on_regions(b) && (st = b->f64 ? build_regions<double>(b) : build_regions<float>(b)) != FI_OK) return st;
+    if (b->regions && (st = b->f64 ? build_regions<double>(b) : build_regions<float>(b)) != FI_OK) return st;
     if (!b->state_on_device) {
         if (b->count() > 0)
             FB_CHECK(cudaMemcpy(b->d_state, b->h_state.data(), sizeof(BState) * b->count(), cudaMemcpyHostToDevice),
@@ -1070,7 +1074,7 @@ fi_status run_rounds(fi_batch *b, const fi_batch_opts *o, int max_rounds, fi_bat
     const int window = o->window > 0 ? o->window : 0;
     const bool use_graph = o->use_graph != 0;
     if (use_graph && *b->h_nactive > 0 &&
-        (!b->graph || b->graph_k != o->ncheck || (on_regions(b) && b->graph_reg != b->h_reg) || b->graph_variant != sweep_kind(b) || b->graph_tol != o->tol ||
+        (!b->graph || b->graph_k != o->ncheck || (b->regions && b->graph_reg != b->h_reg) || b->graph_variant != sweep_kind(b) || b->graph_tol != o->tol ||
          b->graph_window != window || b->graph_max != o->max_iter)) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;

@@ -35,13 +35,13 @@
 // a CTA may leave the cluster at any time.
 //
 // What bounds it.  At 511^3 FP64 DRAM: 1.11 times the field bytes are read (the rings;
-// 64-byte L2 promotion) and the launch takes 4.35 ms, 5.6 TB/s of traffic; FP32 2.7 ms, half
-// DRAM and half instruction issue (53 % active).  Three FP64 CTAs fit an SM (70 KB of slots,
+// 64-byte L2 promotion) and the launch takes 4.25 ms, 5.7 TB/s of traffic; FP32 2.55 ms, bound
+// by instruction issue (78 % active).  Three FP64 CTAs fit an SM (70 KB of slots,
 // 80 registers), 24 warps; a form with 37 slots, two barriers a step, the boundary values
 // applied in passes over the plane and two CTAs per SM took 5.45 and 3.46 ms on the same
 // box.  Small grids are bound by the latency of a step (2.5-3 us alone on an SM), hence
-// the short z-blocks of fused3d_default_variant: 127^3 with walls 240 -> 115 us, 47x33x29
-// 138 -> 11 us.
+// the short z-blocks of fused3d_default_variant and the chained launches: 127^3 with walls
+// 240 -> 98 us, 47x33x29 138 -> 9.3 us, 259x193x125 399 -> 248 us.
 //
 // Double buffering.  Stresses and velocities are read from `in` and written to
 // `out` (distinct buffers), so the pointwise in-place updates of the reference
@@ -78,8 +78,8 @@ namespace {
 // trim flag only marks names: every shape loads the trimmed boxes.  Shapes whose
 // shared memory does not fit a CTA for a precision are not offered for it.
 // fused3d_default_variant picks a 32x8 shape by the grid; the others stay for the
-// autotuner (511^3 FP64 on one box: 32x8 tiles 4.37 ms, 32x16 5.45, 1x4 clusters 4.48;
-// FP32 2.72, 2.86, 2.86 and 64x8 2.98 ms).
+// autotuner (511^3 on one box, before the direct path for ghosts: FP64 32x8 tiles 4.37 ms,
+// 32x16 5.45, 1x4 clusters 4.48; FP32 2.72, 2.86, 2.86 and 64x8 2.98 ms).
 struct Variant {
     int tx, ty, zb, cx, cy, trim;
 };
@@ -293,7 +293,8 @@ bool fused3d_variant_fits(int v, int esz) {
 // zb + 1 steps; with b blocks to each of the 148 SMs a step of all of them takes about
 // 1.25 b + 1.6 us (fitted to FP64 and FP32 runs of 47x33x29 to 511^3: the first term is
 // the throughput of three or four resident CTAs, the second the latency of a step that
-// nothing else hides).  Short blocks pay the extra step, long ones leave SMs idle:
+// nothing else hides).  Short blocks pay the extra step, long ones leave SMs idle (measured
+// before launches were chained and ghosts beside one side had their own path):
 // 259x193x125 FP64 measures 403, 273, 262, 285, 422 us at zb = 1, 8, 16, 32, 128 (the rule
 // takes 16), 127^3 walls 147, 117, 116, 138 at 1, 4, 8, 32 (8), 47x33x29 10, 16, 86 at
 // 1, 4, 32 (1), and 511^3 4.37 and 4.91 ms at 32 and 64 (32, the longest it considers).

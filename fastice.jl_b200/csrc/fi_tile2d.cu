@@ -366,14 +366,15 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
 // next member ahead 67.4), as uniform operands from the constant bank 42.6.
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
 __global__ void __launch_bounds__(RX *RY / PY, MINB)
-    tile2d_batched(const __grid_constant__ Tile2DTable<T> members, const int4 *__restrict__ tiles,
-                   const int *__restrict__ ntiles, int src, int k) {
+    tile2d_batched(const __grid_constant__ Tile2DTable<T> members, int first, bool last, const int4 *__restrict__ tiles,
+                   const int *__restrict__ start, const int *__restrict__ ntiles, int src, int k) {
     extern __shared__ __align__(16) unsigned char t2_smem[];
-    if ((int)blockIdx.x >= *ntiles) return;
-    const int4 d = tiles[blockIdx.x];
+    const int w = start[first] + (int)blockIdx.x;
+    if (w >= (last ? *ntiles : start[first + kTile2DMembers])) return;
+    const int4 d = tiles[w];
     // (a reduction's result is known to be the same in all lanes: the member's values are
     // read as uniform operands)
-    const Tile2DMember<T> &c = members.m[__reduce_max_sync(0xffffffffu, (unsigned)d.x)];
+    const Tile2DMember<T> &c = members.m[__reduce_max_sync(0xffffffffu, (unsigned)(d.x - first))];
     Geom g{};
     KParams p{};
     TConst<T> q{};
@@ -441,8 +442,8 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
 }
 
 template <typename T, bool GF>
-cudaError_t launch_batched_regions(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
-                                   int k, bool chained, cudaStream_t s) {
+cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
+                                   const int *ntiles, int max_tiles, int src, int k, bool chained, cudaStream_t s) {
     using R = Region<T, 32, 32, 2>;
     auto *kern = tile2d_batched<T, 32, 32, 2, 2, GF>;
     int dev = 0;
@@ -463,7 +464,7 @@ cudaError_t launch_batched_regions(const Tile2DTable<T> &members, const int4 *ti
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, members, tiles, ntiles, src, k);
+    return cudaLaunchKernelEx(&cfg, kern, members, first, last, tiles, start, ntiles, src, k);
 }
 
 }  // namespace
@@ -516,17 +517,17 @@ void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty) {
 }
 
 template <typename T>
-cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, const int4 *tiles, const int *ntiles, int max_tiles, int src,
-                                  int k, bool gf, bool chained, cudaStream_t s) {
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
+                                  const int *ntiles, int max_tiles, int src, int k, bool gf, bool chained, cudaStream_t s) {
     if (max_tiles <= 0) return cudaSuccess;
-    return gf ? launch_batched_regions<T, true>(members, tiles, ntiles, max_tiles, src, k, chained, s)
-              : launch_batched_regions<T, false>(members, tiles, ntiles, max_tiles, src, k, chained, s);
+    return gf ? launch_batched_regions<T, true>(members, first, last, tiles, start, ntiles, max_tiles, src, k, chained, s)
+              : launch_batched_regions<T, false>(members, first, last, tiles, start, ntiles, max_tiles, src, k, chained, s);
 }
 
-template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, const int4 *, const int *, int, int, int, bool,
-                                                   bool, cudaStream_t);
-template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, const int4 *, const int *, int, int, int, bool,
-                                                  bool, cudaStream_t);
+template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, int, bool, const int4 *, const int *, const int *, int,
+                                                   int, int, bool, bool, cudaStream_t);
+template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, int, bool, const int4 *, const int *, const int *, int,
+                                                   int, int, bool, bool, cudaStream_t);
 template cudaError_t launch_tile2d<double>(const Geom &, const KParams &, const Ptrs<double> &, const Ptrs<double> &, double *,
                                            int, int, bool, cudaStream_t);
 template cudaError_t launch_tile2d<float>(const Geom &, const KParams &, const Ptrs<float> &, const Ptrs<float> &, float *, int,

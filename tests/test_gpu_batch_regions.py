@@ -67,11 +67,17 @@ def test_more_members_than_a_launch_takes():
     bc.set_variant(0)
     for b in (ba, bc):
         b.advance(6)
-    for q in range(8):  # 62 left: now they fit
+    want, _ = bc.step(max_iter=1 << 30, ncheck=6, tol=0.3, rounds=2)  # some of them retire
+    got, _ = ba.step(max_iter=1 << 30, ncheck=6, tol=0.3, rounds=2)
+    assert [(i["iterations"], i["measure"], i["status"]) for i in got] == [(i["iterations"], i["measure"], i["status"]) for i in want]
+    for q in range(8):  # 62 left: one launch
         ba.remove(a[q])
         bc.remove(c[q])
     for b in (ba, bc):
         b.advance(9)
+    for q in range(8, 70):
+        ba.remove(a[q])
+    ba.advance(4)  # no members: nothing moves
     bad = [(q, f) for q, (x, y) in enumerate(zip(a, c)) for f in F2 if not np.array_equal(x.get_field(f), y.get_field(f))]
     ba.close()
     bc.close()
