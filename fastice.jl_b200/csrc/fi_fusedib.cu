@@ -13,8 +13,8 @@
 // runs one job, and nothing outside the jobs is read or written except as the constant
 // ring of one.
 //
-// Fractions.  They are read from global memory, all of a point's at once and ahead of the
-// wait or barrier before their use, and their lines are brought into the L2 cache two planes
+// Fractions.  They are read from global memory, all of a point's at once (in FP32 ahead of the
+// wait or barrier before their use), and their lines are brought into the L2 cache two planes
 // earlier.  Where every fraction that the updates of an index read is exactly 1 (IBF_FULL:
 // all of the ice except the layers cut by bed and surface) or where nothing is active, none
 // is read and the weights are 1: the masked update is then the plain one bit for bit.
@@ -23,11 +23,12 @@
 // bytes per active FP64 point in dependent loads; one pass without fractions moves 176 and
 // the ring.  After that the code itself is the limit: beyond some 100 KB of it the warps
 // wait for instructions, so there is one body for interior and boundary columns and no
-// second one for unmasked points (FP32, 383^3: 949 us with both, 742 without).  FP64 gets
-// two blocks a multiprocessor: at the 80 registers that three leave, the weights go to local
-// memory, which has no cache beside this much shared memory (1795 us against 1270).
-// Measured per iteration, in place and now: FP64 383^3 1599 -> 1221 us, 191^3 260 -> 214 us;
-// FP32 383^3 1209 -> 717 us, 191^3 215 -> 136 us.
+// second one for unmasked points (FP32, 383^3: 949 us with both, 742 without).  In FP64 it is
+// registers: values spilled to local memory miss every time, as next to no L1 is left beside
+// this much shared memory (36 bytes spilled at three blocks: 2118 us, two blocks 1242).
+// Measured per iteration, in place and now: FP64 383^3 1599 -> 1066 us, 191^3 260 -> 188 us;
+// FP32 383^3 1209 -> 695 us, 191^3 215 -> 129 us; a box a quarter full of ice under rough
+// beds, FP64 383^3 1355-1645 -> 1232-1559 us, 191^3 233-265 -> 166-193 us.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -40,8 +41,6 @@ namespace fi {
 namespace {
 
 constexpr int IX = 32, IY = 8;
-template <typename T>
-constexpr int kMinBlocks = sizeof(T) == 8 ? 2 : Layout<T, IX, IY>::MINB;
 constexpr unsigned IBF_ANY = 0x7fu;
 constexpr unsigned IBF_V_ANY = IBF_V_VCC | IBF_V_CVC | IBF_V_CCV;
 
@@ -210,8 +209,31 @@ __device__ __forceinline__ void ring_masked(const Ctx<T, TX, TY> &c, const KPara
     }
 }
 
-// the plane march of one job
-template <typename T>
+// activity bytes of a point at planes s, s + 1, s + 2
+template <bool PACKED>
+struct PlaneBits {
+    unsigned f0, f1, f2;
+    __device__ __forceinline__ PlaneBits(unsigned a, unsigned b, unsigned c) : f0(a), f1(b), f2(c) {}
+    __device__ __forceinline__ unsigned at0() const { return f0; }
+    __device__ __forceinline__ unsigned at1() const { return f1; }
+    __device__ __forceinline__ unsigned at2() const { return f2; }
+    __device__ __forceinline__ void up(unsigned next) { f0 = f1, f1 = f2, f2 = next; }
+};
+template <>
+struct PlaneBits<true> {
+    unsigned v;
+    __device__ __forceinline__ PlaneBits(unsigned a, unsigned b, unsigned c) : v(a | b << 8 | c << 16) {}
+    __device__ __forceinline__ unsigned at0() const { return v & 0xffu; }
+    __device__ __forceinline__ unsigned at1() const { return v >> 8 & 0xffu; }
+    __device__ __forceinline__ unsigned at2() const { return v >> 16; }
+    __device__ __forceinline__ void up(unsigned next) { v = v >> 8 | next << 16; }
+};
+
+// The plane march of one job.  TIGHT: the fractions and the body force are loaded where they
+// are used instead of ahead of the wait or barrier, and the activity bytes share a register,
+// so that FP64 fits three blocks a multiprocessor at 80 registers (383^3: 1221 us an
+// iteration with two blocks and 120 registers, 1066 so; 191^3 214 and 188.5).
+template <bool TIGHT, typename T>
 __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
                                          const Ptrs<T> &out, const InMaps &maps, uint64_t *bars, unsigned *released, int *err) {
     constexpr int TX = IX, TY = IY, NW = Layout<T, IX, IY>::NW;
@@ -233,11 +255,13 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
     const bool ring = role >= 0 && (role < 2 || lane < TY + (role == 3 ? 1 : 0)) && ri >= 1 && rj >= 1 && ri <= c.n0 + 1 &&
                       rj <= c.n1 + 1;
     const unsigned char *own_bits = in.ibf + c.col(li, lj), *ring_bits = in.ibf + (ring ? c.col(rli, rlj) : 0u);
-    auto bits = [&](const unsigned char *at, bool on, int k) -> unsigned {
-        return on && k >= 1 && k <= c.n2 + 1 ? (unsigned)__ldg(at + c.sxy * k) : 0u;
+    auto bits = [&](const unsigned char *at, int bi, int bj, bool on, int k) -> unsigned {
+        if (!on || k < 1 || k > c.n2 + 1) return 0u;
+        if constexpr (TIGHT) return (unsigned)__ldg(in.ibf + (c.sxy * k + c.col(bi, bj)));
+        return (unsigned)__ldg(at + c.sxy * k);
     };
-    unsigned f0 = bits(own_bits, inside, first), f1 = bits(own_bits, inside, first + 1), f2 = bits(own_bits, inside, first + 2);
-    unsigned r0 = bits(ring_bits, ring, first), r1 = bits(ring_bits, ring, first + 1), r2 = bits(ring_bits, ring, first + 2);
+    PlaneBits<TIGHT> own_at(bits(own_bits, li, lj, inside, first), bits(own_bits, li, lj, inside, first + 1), bits(own_bits, li, lj, inside, first + 2));
+    PlaneBits<TIGHT> ring_at(bits(ring_bits, rli, rlj, ring, first), bits(ring_bits, rli, rlj, ring, first + 1), bits(ring_bits, rli, rlj, ring, first + 2));
     uint32_t phase = 0;
     auto wait_group = [&](int g) -> bool {
         const int b = g % 3;
@@ -250,11 +274,14 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
     bool ok = wait_group(first);
     for (int s = first; s < c.ke && ok; s++, I += c.sxy) {
         c.set_plane(s);
+        const unsigned f0 = own_at.at0(), f1 = own_at.at1(), f2 = own_at.at2();
         const bool own = s >= c.kb;
         const int zf = z_fixed(c, p, s + 1);
         if (s <= c.n2) {
             const bool any = (f0 | f1) & IBF_ANY;
-            const StressW<T> sw = stress_w(in, I, c.sx, c.sxy, any && !(f0 & f1 & IBF_FULL));
+            const bool need = any && !(f0 & f1 & IBF_FULL);
+            StressW<T> sw;
+            if constexpr (!TIGHT) sw = stress_w(in, I, c.sx, c.sxy, need);
             if ((f2 & IBF_ANY) && !(f2 & IBF_FULL)) {
                 const long long N = I + 2 * c.sxy;
                 for (int w : {W_CCC, W_VVC, W_VCV, W_CVV}) prefetch_l2(in.wna[w] + N);
@@ -263,6 +290,7 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
             ok = wait_group(s + 1);
             if (!ok) break;
             if (__any_sync(0xffffffffu, any)) {
+                if constexpr (TIGHT) sw = stress_w(in, I, c.sx, c.sxy, need);
                 const Centre<T> v = centre_masked<F_P | F_XX | F_YY | F_ZZ>(c, p, q, in, li, lj, I, sw, f0 & IBF_S_CCC);
                 const T xy = xy_masked(c, q, li, lj, sw, f0 & IBF_S_VVC);
                 const T xz = xz_masked(c, q, li, lj, sw, f1 & IBF_S_VCV), yz = yz_masked(c, q, li, lj, sw, f1 & IBF_S_CVV);
@@ -276,7 +304,7 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
                     k.zzm = tv - k.zz;
                 }
             }
-            if (ring) ring_masked(c, p, q, in, out, s, zf, own, role, rli, rlj, r0, r1);
+            if (ring) ring_masked(c, p, q, in, out, s, zf, own, role, rli, rlj, ring_at.at0(), ring_at.at1());
         } else if (inside && p.bc_kind[2][1] == FI_BC_TRACTION) {
             // the top plane of vertices has no stresses: the ghosts over a traction top
             const T tv = T(2.0) * q.bc_val[2][1][2];
@@ -288,25 +316,34 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
             }
         }
         if (own) {
-            T gx = q.g_val[0], gy = q.g_val[1], gz = q.g_val[2];
-            if (inside) {
-                gx = body_force(p, q, in.gx, 0, I);
-                gy = body_force(p, q, in.gy, 1, I);
-                gz = body_force(p, q, in.gz, 2, I);
+            const bool need = (f0 & IBF_V_ANY) && !(f0 & IBF_FULL);
+            const bool unit = __all_sync(0xffffffffu, !need);
+            VelocityW<T> vw;
+            T g[3];
+            auto force = [&](const T *field, int d) {
+                return TIGHT ? (inside ? body_force(p, q, field, d, I) : q.g_val[d]) : g[d];
+            };
+            if constexpr (!TIGHT) {
+                g[0] = q.g_val[0], g[1] = q.g_val[1], g[2] = q.g_val[2];
+                if (inside) {
+                    g[0] = body_force(p, q, in.gx, 0, I);
+                    g[1] = body_force(p, q, in.gy, 1, I);
+                    g[2] = body_force(p, q, in.gz, 2, I);
+                }
+                vw = velocity_w(in, I, c.sx, c.sxy, need);
             }
-            const VelocityW<T> vw = velocity_w(in, I, c.sx, c.sxy, (f0 & IBF_V_ANY) && !(f0 & IBF_FULL));
-            const bool unit = __all_sync(0xffffffffu, vw.nx == T(1) && vw.ny == T(1) && vw.nz == T(1));
             __syncthreads();
-            const T vx = vx_masked(c, q, li, lj, vw, f0 & IBF_V_VCC, unit, gx);
-            const T vy = vy_masked(c, q, li, lj, vw, f0 & IBF_V_CVC, unit, gy);
-            const T vz = vz_masked(c, q, li, lj, vw, f0 & IBF_V_CCV, unit, gz, k);
+            if constexpr (TIGHT) vw = velocity_w(in, I, c.sx, c.sxy, need);
+            const T vx = vx_masked(c, q, li, lj, vw, f0 & IBF_V_VCC, unit, force(in.gx, 0));
+            const T vy = vy_masked(c, q, li, lj, vw, f0 & IBF_V_CVC, unit, force(in.gy, 1));
+            const T vz = vz_masked(c, q, li, lj, vw, f0 & IBF_V_CCV, unit, force(in.gz, 2), k);
             v_store<true, true>(c, p, q, in, out, s, li, lj, fl, I, k, vx, vy, vz);
         }
         k.Pm = k.P;
         k.zzm = k.zz;
         k.etm = *EL(M_ET, c.V0);
-        f0 = f1, f1 = f2, f2 = bits(own_bits, inside, s + 3);
-        r0 = r1, r1 = r2, r2 = bits(ring_bits, ring, s + 3);
+        own_at.up(bits(own_bits, li, lj, inside, s + 3));
+        ring_at.up(bits(ring_bits, rli, rlj, ring, s + 3));
         __syncwarp();
         if (s + 3 <= gmax && lane == 0) {
             unsigned n;
@@ -323,7 +360,7 @@ __device__ __forceinline__ void sweep_ib(Ctx<T, IX, IY> &c, const KParams &p, co
 }
 
 // one job: x = tile x | tile y << 16, y = kb, z = ke
-template <typename T>
+template <bool TIGHT, typename T>
 __device__ __forceinline__ void run_job(const Geom &g, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
                                         const Ptrs<T> &out, const InMaps &maps, unsigned char *smem, int4 job, int *err) {
     using Lay = Layout<T, IX, IY>;
@@ -348,21 +385,22 @@ __device__ __forceinline__ void run_job(const Geom &g, const KParams &p, const T
     c.sxy = g.sxy;
     c.hx0 = c.hx1 = c.hy0 = c.hy1 = false;
     chain_launches();
-    sweep_ib(c, p, q, in, out, maps, bars, released, err);
+    sweep_ib<TIGHT>(c, p, q, in, out, maps, bars, released, err);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(Layout<T, IX, IY>::NT, kMinBlocks<T>)
+__global__ void __launch_bounds__(Layout<T, IX, IY>::NT, Layout<T, IX, IY>::MINB)
     fusedib_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, const __grid_constant__ InMaps maps,
                    const int4 *__restrict__ jobs, int *err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    run_job(g, p, q, in, out, maps, smem_raw, jobs[blockIdx.x], err);
+    run_job<sizeof(T) == 8>(g, p, q, in, out, maps, smem_raw, jobs[blockIdx.x], err);
 }
 
 // jobs of several models: w = member; the block copies its member's parameters and pointers
-// into shared memory (e: the roles of its buffers)
+// into shared memory (e: the roles of its buffers).  With them there, FP64 at three blocks a
+// multiprocessor spills (12 glaciers of 16^3-48^3: 71 us an iteration against 63 at two).
 template <typename T>
-__global__ void __launch_bounds__(Layout<T, IX, IY>::NT, kMinBlocks<T>)
+__global__ void __launch_bounds__(Layout<T, IX, IY>::NT, sizeof(T) == 8 ? 2 : Layout<T, IX, IY>::MINB)
     fusedib_batched(const IbFusedMember<T> *__restrict__ members, const int4 *__restrict__ jobs, int e) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(16) IbFusedHead<T> sm;
@@ -372,7 +410,7 @@ __global__ void __launch_bounds__(Layout<T, IX, IY>::NT, kMinBlocks<T>)
     unsigned *dst = reinterpret_cast<unsigned *>(&sm);
     for (int w = threadIdx.x; w < (int)(sizeof(IbFusedHead<T>) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
     __syncthreads();
-    run_job(sm.g, sm.p, sm.q, sm.f[e], sm.f[2 + e], reinterpret_cast<const InMaps &>(m.maps[e]), smem_raw, job, sm.err);
+    run_job<false>(sm.g, sm.p, sm.q, sm.f[e], sm.f[2 + e], reinterpret_cast<const InMaps &>(m.maps[e]), smem_raw, job, sm.err);
 }
 
 // 1 where a tile column has, in this plane, a point next to an active one (or active)
