@@ -37,16 +37,14 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 
 # DRAM bytes per cell of one fused-sweep launch: dram__bytes_read.sum +
-# dram__bytes_write.sum of one ncu-captured 255^3 launch (32x8 tiles, z-blocks of
-# 32, summarised in profiles/fused3d_slab255_ncu_full.md, v6) divided by its cell
-# count; traffic grows with the cell count, so it scales to 511^3.
-TRAFFIC_BYTES_PER_CELL = {"f64": 233.3, "f32": None}
-# DRAM bytes per cell of one steady-state immersed-boundary iteration (update_σ!,
-# update_V! and their six boundary launches, inactive zeros no longer stored,
-# block list in use): dram__bytes_read.sum + dram__bytes_write.sum of one
-# ncu-captured iteration of the 191^3 glacier divided by its cell count
-# (profiles/ib_glacier191_dram.md); the same geometry scales to 383^3.
-IB_TRAFFIC_BYTES_PER_CELL = {"f64": 109.5, "f32": 74.9}
+# dram__bytes_write.sum of one ncu-captured launch (511x511x63 FP64, 511x511x95
+# FP32, 32x8 tiles, z-blocks of 32, summarised in profiles/fused3d_march_ncu.md)
+# divided by its cell count; traffic grows with the cell count, so it scales to 511^3.
+TRAFFIC_BYTES_PER_CELL = {"f64": 185.7, "f32": 93.2}
+# DRAM bytes per cell of one fused immersed-boundary sweep: dram__bytes_read.sum +
+# dram__bytes_write.sum of one ncu-captured launch of the 191^3 glacier divided by its
+# cell count (profiles/fusedib_glacier191_ncu.md); the same geometry scales to 383^3.
+IB_TRAFFIC_BYTES_PER_CELL = {"f64": 102.9, "f32": 55.6}
 
 
 def load_fastice():
@@ -342,8 +340,8 @@ def _base_line(metric, value, unit, steps, warmup, ms, dtype, cfg, hib=True):
 def run_batched(args):
     """Batched 2D solves: `instances` pure-shear inclusion problems (seeds 0..k-1,
     63-511 cells per side, 1-16 inclusions, contrasts up to 1e4) in one batch:
-    autotuned tile shape, CUDA-graph replay of each check round, one step = one
-    check round.  With --storage f32 (the default) every PT sweep runs on FP32
+    launches of several iterations, CUDA-graph replay of each check round, one step =
+    one check round (the one-iteration sweeps' tile heights are timed beside it).  With --storage f32 (the default) every PT sweep runs on FP32
     storage inside a per-member FP64 defect correction (FP64 solution and
     residuals) to the FP64 measure --tol (1e-6); --storage f64 runs plain FP64
     sweeps.  value = instances solved / wall time of the solve.  The same method
@@ -383,7 +381,6 @@ def run_batched(args):
     for q in range(min(args.alone, len(models))):
         mq = members([q])
         b1 = fi.BatchedStokes2D(mq)
-        b1.set_variant(best)
         it1, s1 = b1.solve(max_iter=max_iter, ncheck=ncheck, tol=tol, window=window, use_graph=True, mode=mode)
         b1.close()
         mq[0].close()
@@ -426,7 +423,8 @@ def run_batched(args):
                  "one_at_a_time": alone,
                  "speedup_vs_one_at_a_time": (done / sec) / alone["solves_per_s"] if alone["solves_per_s"] else None,
                  "error_vs_fp64_solve": errs,
-                 "gpu_launches": "k sweeps + 4 bookkeeping kernels per check round, replayed as one graph; per outer "
+                 "gpu_launches": "a launch per 64 members and four iterations + 6 bookkeeping kernels per check round, replayed as "
+                                 "one graph; per outer "
                                  "step of the defect correction a few FP64 kernels per member"})
     return line
 
@@ -650,7 +648,7 @@ def run_glacier(args):
     traffic = tr * n * n * n if tr else None
     dram = traffic / (d0["ms_per_step"] / 1e3) / 1e9 if traffic else None
     line.update({"kernel_path": d0["path"],
-                 "gpu_launches": 8 * args.steps,  # update_σ!, update_V! and six boundary launches per iteration
+                 "gpu_launches": args.steps,  # one fused sweep per iteration
                  "roofline": {"bound": "hbm", "achieved": d0["teff_gbs"], "peak": peak, "unit": "GB/s",
                               "frac": d0["teff_gbs"] / peak, "peak_source": peak_kind,
                               "algorithmic_bytes": A * (8 if dt0 == "f64" else 4), "traffic": traffic,
@@ -828,9 +826,8 @@ def run_shapes(args):
 def run_ibbatch(args):
     """3D immersed-boundary glaciers of uneven sizes (seeded beds, n^3 with n drawn
     uniformly from --sizes, 48 to 160 by default) advanced together by shared launches (BatchedIB3D:
-    eight launches per iteration of all members, iteration pairs replayed as a CUDA
-    graph) against the same models advanced one at a time (each model's own
-    graph-replayed iterations, synchronised before the next model).  One step = one
+    one fused launch per iteration of all members) against the same models advanced
+    one at a time (each model's own sweeps, synchronised before the next model).  One step = one
     PT iteration of every member; value = member iterations per second of the
     batch, wall time around the advance and a synchronize, after warm-up."""
     fi = load_fastice()
@@ -875,7 +872,7 @@ def run_ibbatch(args):
                                    "seconds": res["one_at_a_time_s"]},
                  "speedup_vs_one_at_a_time": res["one_at_a_time_s"] / res["batched_s"],
                  "teff_gbs_36_pass": teff_bytes * K / res["batched_s"] / 1e9,
-                 "gpu_launches": f"{8 * K} (eight per iteration of all members; graph-replayed pairs)"})
+                 "gpu_launches": f"{K} (one per iteration of all members)"})
     return line
 
 
