@@ -444,7 +444,7 @@ fi_status reference_pairs(fi_model *m, int pairs) {
 // viscosity of the iteration before, as after the reference's swap.
 template <typename T>
 fi_status tile2d_advance(fi_model *m, int niter) {
-    const Tile2DPlan plan = tile2d_plan(m->g);
+    const Tile2DPlan plan = tile2d_plan(m->g.n[0], m->g.n[1]);
     const int pairs = (niter + 2 * plan.k - 1) / (2 * plan.k), L = 2 * pairs;
     for (int l = 0; l < L; l++) {
         const int k = (int)((long long)niter * (l + 1) / L - (long long)niter * l / L);

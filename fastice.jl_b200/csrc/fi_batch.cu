@@ -831,12 +831,10 @@ fi_status build_tiles(fi_batch *b, int ty) {
 // 31^2-63^2 in FP32 2.5 / 2.1 at k = 4 / 10.
 int region_depth(const fi_batch *b) {
     auto tiles = [&](int k) {
+        const int side = tile2d_batch_tile(k);
         long long t = 0;
-        for (const fi_model *m : b->models) {
-            int tx, ty;
-            tile2d_member_tile(m->d.grid.n[0], m->d.grid.n[1], k, &tx, &ty);
-            t += (long long)((m->d.grid.n[0] + tx) / tx) * ((m->d.grid.n[1] + ty) / ty);
-        }
+        for (const fi_model *m : b->models)
+            t += (long long)t2_tiles(m->d.grid.n[0], side, false) * t2_tiles(m->d.grid.n[1], side, false);
         return t;
     };
     for (int k = 10; k > 4; k--)
@@ -854,12 +852,10 @@ fi_status build_regions(fi_batch *b) {
         std::vector<int4> all;
         std::vector<int> first(n), cnt(n);
         for (int q = 0; q < n; q++) {
-            const int *c = b->models[q]->d.grid.n;
-            int tx, ty;
-            tile2d_member_tile(c[0], c[1], b->reg_k, &tx, &ty);
+            const int *c = b->models[q]->d.grid.n, side = tile2d_batch_tile(b->reg_k);
             first[q] = (int)all.size();
-            for (int y = 0; y < (c[1] + ty) / ty; y++)
-                for (int x = 0; x < (c[0] + tx) / tx; x++) all.push_back(make_int4(q, x, y, 0));
+            for (int y = 0; y < t2_tiles(c[1], side, false); y++)
+                for (int x = 0; x < t2_tiles(c[0], side, false); x++) all.push_back(make_int4(q, x, y, 0));
             cnt[q] = (int)all.size() - first[q];
         }
         const int tot = (int)all.size();
@@ -896,7 +892,7 @@ fi_status build_regions(fi_batch *b) {
         const BInst<T> &v = reinterpret_cast<const BInst<T> *>(b->h_inst.data())[q];
         Tile2DMember<T> &u = tab[q / kTile2DMembers].m[q % kTile2DMembers];
         u.n[0] = v.n0, u.n[1] = v.n1, u.pitch = (int)v.pitch, u.forced = v.pforce;
-        tile2d_member_tile(v.n0, v.n1, b->reg_k, &u.tx, &u.ty);
+        for (int d = 0; d < 2; d++) u.shift[d] = t2_shift(u.n[d], tile2d_batch_tile(b->reg_k), false);
         std::memcpy(u.bc_kind, v.bc_kind, sizeof(u.bc_kind));
         std::memcpy(u.bc_val, v.bc_val, sizeof(u.bc_val));
         u.inv_dx[0] = v.idx, u.inv_dx[1] = v.idy, u.dt_P = v.dtP;
@@ -930,7 +926,7 @@ cudaError_t launch_regions(fi_batch *b, bool all, int k) {
         left -= step;
         for (int c = 0; c < groups && e == cudaSuccess; c++)
             e = launch_tile2d_batched<T>(tab[c], c * kTile2DMembers, c == groups - 1, list, start, nt, b->reg_max[c], l & 1, step,
-                                         b->reg_gf, l + c > 0, b->stream);
+                                         tile2d_batch_tile(b->reg_k), b->reg_gf, l + c > 0, b->stream);
     }
     return e;
 }

@@ -17,6 +17,7 @@
 #include <string>
 
 #include "../../include/fastice_b200.h"
+#include "fi_tile2d_map.h"
 
 namespace fi {
 
@@ -222,11 +223,6 @@ bool fused3d_variant_fits(int v, int esz);
 const char *fused3d_variant_name(int v);
 
 // ---- several 2D iterations in one launch (fi_tile2d.cu) ----
-struct Tile2DPlan {
-    int shape;  // region shape
-    int k;      // most iterations of one launch
-};
-Tile2DPlan tile2d_plan(const Geom &g);
 // k iterations: P, τ, V, η read from `in`, written to `out` (distinct buffers, ghosts
 // included); with write_prev, η before the last of them to eta_prev (interior).  η is
 // read only when frozen.
@@ -238,7 +234,7 @@ cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, co
 // needs of a member; f[src] is read, f[src ^ 1] written (P, τxx, τyy, τxy, V.x, V.y); η fixed.
 template <typename T>
 struct Tile2DMember {
-    int n[2], tx, ty;  // cells; the member's tile (tile2d_member_tile)
+    int n[2], shift[2];  // cells; t2_shift of the tiles
     int pitch, forced, bc_kind[2][2], g_kind[2];
     T inv_dx[2], dt_P, dt_tau[3], dt_V[2], g_val[2], bc_val[2][2][2];
     const T *eta, *gx, *gy, *fP;
@@ -250,15 +246,15 @@ template <typename T>
 struct Tile2DTable {
     Tile2DMember<T> m[kTile2DMembers];
 };
-// tile sides of an n0 x n1 grid for launches of at most k iterations
-void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty);
+// sides of the tiles for launches of at most k iterations
+constexpr int tile2d_batch_tile(int k) { return 32 - 2 * k; }
 // The regions of the members first .. first + kTile2DMembers - 1 (members holds those): items
 // start[first] .. of the list, up to the next group's or the list's end (last:
 // no group follows).  gf: some member's body force is a field; chained: right after another of these
 // launches.
 template <typename T>
 cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                  const int *ntiles, int max_tiles, int src, int k, bool gf, bool chained, cudaStream_t s);
+                                  const int *ntiles, int max_tiles, int src, int k, int tile, bool gf, bool chained, cudaStream_t s);
 
 // ---- mixed-precision solve helpers (fi_mixed.cu) ----
 template <typename S, typename D>

@@ -56,6 +56,7 @@ struct Region {
 struct TileArgs {
     int k;           // iterations of this launch
     int tx, ty;      // inner tile
+    int x0, y0;      // first position of the first region
     int write_prev;  // the last launch of an advance: also write η of the iteration before
 };
 
@@ -236,7 +237,7 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
     const int n0 = g.n[0], n1 = g.n[1];
     // (a batch has no periodic members)
     const bool px = !BATCH && p.bc_kind[0][0] == FI_BC_PERIODIC, py = !BATCH && p.bc_kind[1][0] == FI_BC_PERIODIC;
-    const int i0 = 1 + bx * ta.tx - ta.k, j0 = 1 + by * ta.ty - ta.k;
+    const int i0 = ta.x0 + bx * ta.tx, j0 = ta.y0 + by * ta.ty;
     const int gi = i0 + x;
     const int a0 = (y0 + 1) * PW + x + 1;
     const bool edge = (!px && (i0 <= 1 || i0 + RX > n0)) || (!py && (j0 <= 1 || j0 + RY > n1));
@@ -314,14 +315,9 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- the inner tile (with the ghosts beside it) to the other buffer ----
-    const int xe = px ? n0 : n0 + 1, ye = py ? n1 : n1 + 1;  // last position that tiles own
     const int bx0 = i0 + ta.k, by0 = j0 + ta.k;
     const auto &P = v.P, &xx = v.xx, &yy = v.yy, &xy = v.xy, &vx = v.vx, &vy = v.vy, &et = v.et;
-    auto owned = [](int gq, int b, int t, int last, bool per) {
-        if (gq >= b && gq < b + t && gq <= last) return true;
-        return !per && ((gq == 0 && b == 1) || (gq == last + 1 && last >= b && last < b + t));
-    };
-    if (!owned(gi, bx0, ta.tx, xe, px)) return;
+    if (!t2_owned(gi, bx0, ta.tx, n0, px)) return;
     // periodic images of centre (c) and vertex (v) values along a dimension: 0 = none
     auto image_c = [](int gq, int n, bool per) { return !per ? 0 : gq == n ? -n : gq == 1 ? n : 0; };
     auto image_v = [](int gq, int n, bool per) { return !per ? 0 : gq == n ? -n : gq <= 2 ? n : 0; };
@@ -329,7 +325,7 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
 #pragma unroll
     for (int r = 0; r < PY; r++) {
         const int gj = j0 + y0 + r;
-        if (!owned(gj, by0, ta.ty, ye, py)) continue;
+        if (!t2_owned(gj, by0, ta.ty, n1, py)) continue;
         const int a = a0 + r * PW;
         const long long I = (long long)gi + g.pitch * (long long)gj;
         const long long yc = g.pitch * image_c(gj, n1, py), yv = g.pitch * image_v(gj, n1, py);
@@ -367,7 +363,7 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
 __global__ void __launch_bounds__(RX *RY / PY, MINB)
     tile2d_batched(const __grid_constant__ Tile2DTable<T> members, int first, bool last, const int4 *__restrict__ tiles,
-                   const int *__restrict__ start, const int *__restrict__ ntiles, int src, int k) {
+                   const int *__restrict__ start, const int *__restrict__ ntiles, int src, int k, int tile) {
     extern __shared__ __align__(16) unsigned char t2_smem[];
     const int w = start[first] + (int)blockIdx.x;
     if (w >= (last ? *ntiles : start[first + kTile2DMembers])) return;
@@ -400,15 +396,8 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
     const int dst = src ^ 1;
     out.P = c.f[dst][0], out.txx = c.f[dst][1], out.tyy = c.f[dst][2], out.txy = c.f[dst][3], out.Vx = c.f[dst][4],
     out.Vy = c.f[dst][5];
-    const TileArgs ta{k, c.tx, c.ty, 0};
+    const TileArgs ta{k, tile, tile, 1 - k - c.shift[0], 1 - k - c.shift[1], 0};
     run_region<T, RX, RY, PY, GF, true>(g, p, q, in, out, nullptr, ta, d.y, d.z, t2_smem);
-}
-
-// No tile starts at the last node of a bounded dimension: the ghosts there follow from the
-// cell before it, which would lie outside what the region gets right.
-int inner_tile(int t, int n, bool per) {
-    while (!per && t > 2 && n % t == 0) t--;
-    return t;
 }
 
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
@@ -425,10 +414,10 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
         attr_set[dev] = true;
     }
     const bool px = p.bc_kind[0][0] == FI_BC_PERIODIC, py = p.bc_kind[1][0] == FI_BC_PERIODIC;
-    const int ex = px ? g.n[0] : g.n[0] + 1, ey = py ? g.n[1] : g.n[1] + 1;
-    const TileArgs ta{k, inner_tile(RX - 2 * k, g.n[0], px), inner_tile(RY - 2 * k, g.n[1], py), write_prev ? 1 : 0};
+    const TileArgs ta{k, RX - 2 * k, RY - 2 * k, 1 - k - t2_shift(g.n[0], RX - 2 * k, px),
+                      1 - k - t2_shift(g.n[1], RY - 2 * k, py), write_prev ? 1 : 0};
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((ex + ta.tx - 1) / ta.tx, (ey + ta.ty - 1) / ta.ty);
+    cfg.gridDim = dim3(t2_tiles(g.n[0], ta.tx, px), t2_tiles(g.n[1], ta.ty, py));
     cfg.blockDim = dim3(R::NT);
     cfg.dynamicSmemBytes = R::SMEM;
     cfg.stream = s;
@@ -443,7 +432,7 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
 
 template <typename T, bool GF>
 cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                   const int *ntiles, int max_tiles, int src, int k, bool chained, cudaStream_t s) {
+                                   const int *ntiles, int max_tiles, int src, int k, int tile, bool chained, cudaStream_t s) {
     using R = Region<T, 32, 32, 2>;
     auto *kern = tile2d_batched<T, 32, 32, 2, 2, GF>;
     int dev = 0;
@@ -464,34 +453,10 @@ cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, boo
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, members, first, last, tiles, start, ntiles, src, k);
+    return cudaLaunchKernelEx(&cfg, kern, members, first, last, tiles, start, ntiles, src, k, tile);
 }
 
 }  // namespace
-
-// Region shapes: 0 = 32 x 16, one row a thread, one CTA per SM; 1 = 32 x 32, two rows, one;
-// 2 = 32 x 32, two rows, two CTAs per SM (64 registers).
-//
-// A launch costs about 4 us that k iterations share (launch, first loads, last stores);
-// deeper launches recompute more.  While the tiles of a shape fit the SMs at once, the
-// deepest such launch is best, on the smaller region (an iteration of it takes 0.5 us
-// against 1.6): FP64 us per iteration, reference-shaped -> chosen (others): 128^2
-// 13.8 -> 1.37 at 32x16 k = 5 (k = 3: 1.73; 32x32 k = 10: 1.91); 200^2 2.37 at 32x32
-// k = 6 (32x16 k = 2: 2.27, k = 4: 2.81); 300x240 2.67 at k = 4 (k = 3: 2.98).  Beyond that
-// two CTAs per SM hide each other's loads: 1021x509 21.9 -> 10.98 at k = 4 (k = 3 11.2,
-// k = 2 12.2, one CTA per SM 12.1), FP32 7.8 (9.1); 1224x1000 24.0, FP32 15.9.
-Tile2DPlan tile2d_plan(const Geom &g) {
-    auto tiles = [&](int rx, int ry, int k) {
-        const long long tx = rx - 2 * k, ty = ry - 2 * k;
-        return ((g.n[0] + tx) / tx) * ((g.n[1] + ty) / ty);
-    };
-    constexpr int kSMs = 148;
-    for (int k = 6; k >= 3; k--)
-        if (tiles(32, 16, k) <= kSMs) return {0, k};
-    for (int k = 10; k >= 4; k--)
-        if (tiles(32, 32, k) <= kSMs) return {1, k};
-    return {2, 4};
-}
 
 template <typename T, bool GF>
 static cudaError_t launch_shape(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, T *eta_prev, int shape,
@@ -511,23 +476,18 @@ cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, co
               : launch_shape<T, false>(g, p, in, out, eta_prev, shape, k, write_prev, s);
 }
 
-void tile2d_member_tile(int n0, int n1, int k, int *tx, int *ty) {
-    *tx = inner_tile(32 - 2 * k, n0, false);
-    *ty = inner_tile(32 - 2 * k, n1, false);
-}
-
 template <typename T>
 cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                  const int *ntiles, int max_tiles, int src, int k, bool gf, bool chained, cudaStream_t s) {
+                                  const int *ntiles, int max_tiles, int src, int k, int tile, bool gf, bool chained, cudaStream_t s) {
     if (max_tiles <= 0) return cudaSuccess;
-    return gf ? launch_batched_regions<T, true>(members, first, last, tiles, start, ntiles, max_tiles, src, k, chained, s)
-              : launch_batched_regions<T, false>(members, first, last, tiles, start, ntiles, max_tiles, src, k, chained, s);
+    return gf ? launch_batched_regions<T, true>(members, first, last, tiles, start, ntiles, max_tiles, src, k, tile, chained, s)
+              : launch_batched_regions<T, false>(members, first, last, tiles, start, ntiles, max_tiles, src, k, tile, chained, s);
 }
 
 template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, int, bool, const int4 *, const int *, const int *, int,
-                                                   int, int, bool, bool, cudaStream_t);
+                                                   int, int, int, bool, bool, cudaStream_t);
 template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, int, bool, const int4 *, const int *, const int *, int,
-                                                   int, int, bool, bool, cudaStream_t);
+                                                   int, int, int, bool, bool, cudaStream_t);
 template cudaError_t launch_tile2d<double>(const Geom &, const KParams &, const Ptrs<double> &, const Ptrs<double> &, double *,
                                            int, int, bool, cudaStream_t);
 template cudaError_t launch_tile2d<float>(const Geom &, const KParams &, const Ptrs<float> &, const Ptrs<float> &, float *, int,
