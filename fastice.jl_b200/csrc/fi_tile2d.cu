@@ -366,7 +366,12 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
                    const int *__restrict__ start, const int *__restrict__ ntiles, int src, int k, int tile) {
     extern __shared__ __align__(16) unsigned char t2_smem[];
     const int w = start[first] + (int)blockIdx.x;
-    if (w >= (last ? *ntiles : start[first + kTile2DMembers])) return;
+    if (w >= (last ? *ntiles : start[first + kTile2DMembers])) {
+        // Also a block without work waits: a group with no active member would otherwise be a
+        // grid that ends at once, and the launch chained to it would run beside the one before.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        return;
+    }
     const int4 d = tiles[w];
     // (a reduction's result is known to be the same in all lanes: the member's values are
     // read as uniform operands)
