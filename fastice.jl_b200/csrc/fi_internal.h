@@ -248,13 +248,12 @@ struct Tile2DTable {
 };
 // sides of the tiles for launches of at most k iterations
 constexpr int tile2d_batch_tile(int k) { return 32 - 2 * k; }
-// The regions of the members first .. first + kTile2DMembers - 1 (members holds those): items
-// start[first] .. of the list, up to the next group's or the list's end (last:
-// no group follows).  gf: some member's body force is a field; chained: right after another of these
-// launches.
+// The regions of the members first .. end - 1 (members holds those): items start[first] ..
+// start[end] - 1 of the list, a block each; there may be more blocks than items.  gf: some
+// member's body force is a field; chained: right after another of these launches.
 template <typename T>
-cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                  const int *ntiles, int max_tiles, int src, int k, int tile, bool gf, bool chained, cudaStream_t s);
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, int end, const int4 *tiles, const int *start,
+                                  int blocks, int src, int k, int tile, bool gf, bool chained, cudaStream_t s);
 
 // ---- mixed-precision solve helpers (fi_mixed.cu) ----
 template <typename S, typename D>

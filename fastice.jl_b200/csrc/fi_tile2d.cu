@@ -362,11 +362,11 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
 // next member ahead 67.4), as uniform operands from the constant bank 42.6.
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
 __global__ void __launch_bounds__(RX *RY / PY, MINB)
-    tile2d_batched(const __grid_constant__ Tile2DTable<T> members, int first, bool last, const int4 *__restrict__ tiles,
-                   const int *__restrict__ start, const int *__restrict__ ntiles, int src, int k, int tile) {
+    tile2d_batched(const __grid_constant__ Tile2DTable<T> members, int first, int end, const int4 *__restrict__ tiles,
+                   const int *__restrict__ start, int src, int k, int tile) {
     extern __shared__ __align__(16) unsigned char t2_smem[];
     const int w = start[first] + (int)blockIdx.x;
-    if (w >= (last ? *ntiles : start[first + kTile2DMembers])) {
+    if (w >= start[end]) {
         // Also a block without work waits: a group with no active member would otherwise be a
         // grid that ends at once, and the launch chained to it would run beside the one before.
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -436,8 +436,8 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
 }
 
 template <typename T, bool GF>
-cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                   const int *ntiles, int max_tiles, int src, int k, int tile, bool chained, cudaStream_t s) {
+cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, int end, const int4 *tiles, const int *start,
+                                   int blocks, int src, int k, int tile, bool chained, cudaStream_t s) {
     using R = Region<T, 32, 32, 2>;
     auto *kern = tile2d_batched<T, 32, 32, 2, 2, GF>;
     int dev = 0;
@@ -449,7 +449,7 @@ cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, boo
         attr_set[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(max_tiles);
+    cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(R::NT);
     cfg.dynamicSmemBytes = R::SMEM;
     cfg.stream = s;
@@ -458,7 +458,7 @@ cudaError_t launch_batched_regions(const Tile2DTable<T> &members, int first, boo
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, members, first, last, tiles, start, ntiles, src, k, tile);
+    return cudaLaunchKernelEx(&cfg, kern, members, first, end, tiles, start, src, k, tile);
 }
 
 }  // namespace
@@ -482,17 +482,16 @@ cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, co
 }
 
 template <typename T>
-cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, bool last, const int4 *tiles, const int *start,
-                                  const int *ntiles, int max_tiles, int src, int k, int tile, bool gf, bool chained, cudaStream_t s) {
-    if (max_tiles <= 0) return cudaSuccess;
-    return gf ? launch_batched_regions<T, true>(members, first, last, tiles, start, ntiles, max_tiles, src, k, tile, chained, s)
-              : launch_batched_regions<T, false>(members, first, last, tiles, start, ntiles, max_tiles, src, k, tile, chained, s);
+cudaError_t launch_tile2d_batched(const Tile2DTable<T> &members, int first, int end, const int4 *tiles, const int *start,
+                                  int blocks, int src, int k, int tile, bool gf, bool chained, cudaStream_t s) {
+    return gf ? launch_batched_regions<T, true>(members, first, end, tiles, start, blocks, src, k, tile, chained, s)
+              : launch_batched_regions<T, false>(members, first, end, tiles, start, blocks, src, k, tile, chained, s);
 }
 
-template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, int, bool, const int4 *, const int *, const int *, int,
-                                                   int, int, int, bool, bool, cudaStream_t);
-template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, int, bool, const int4 *, const int *, const int *, int,
-                                                   int, int, int, bool, bool, cudaStream_t);
+template cudaError_t launch_tile2d_batched<double>(const Tile2DTable<double> &, int, int, const int4 *, const int *, int, int, int,
+                                                   int, bool, bool, cudaStream_t);
+template cudaError_t launch_tile2d_batched<float>(const Tile2DTable<float> &, int, int, const int4 *, const int *, int, int, int,
+                                                  int, bool, bool, cudaStream_t);
 template cudaError_t launch_tile2d<double>(const Geom &, const KParams &, const Ptrs<double> &, const Ptrs<double> &, double *,
                                            int, int, bool, cudaStream_t);
 template cudaError_t launch_tile2d<float>(const Geom &, const KParams &, const Ptrs<float> &, const Ptrs<float> &, float *, int,

@@ -60,3 +60,28 @@ def test_empty_groups(use_graph):
     assert set(status[:GROUP]) == {"active"} and set(status[GROUP:]) == {"converged"}, status
     assert got == want
     assert all(np.array_equal(x, y) and np.isfinite(y).all() for x, y in zip(state, state_w))
+
+
+@pytest.mark.parametrize("use_graph", [True, False], ids=["graph", "launches"])
+def test_solve_again(use_graph):
+    # launches follow the retirements; the next solve starts with all members again
+    fi = load_fastice()
+    out = []
+    for plain in (True, False):
+        models = [_model(fi, q, q % 3 == 1 or q > GROUP) for q in range(GROUP + 9)]
+        b = fi.BatchedStokes2D(models)
+        if plain:
+            b.set_variant(0)
+        items = []
+        for tol in (5e-2, 2e-2, 1e-2):
+            items += b.solve(max_iter=3000, ncheck=50, tol=tol, use_graph=use_graph)[0]
+            for q in (2, 5, GROUP + 3):
+                models[q].set_field("Vx", 0.3 + models[q].get_field("Vx"))
+        out.append(([(i["iterations"], i["measure"], i["status"]) for i in items], [m.get_field(f) for m in models for f in F2]))
+        b.close()
+        for m in models:
+            m.close()
+    (want, state_w), (got, state) = out
+    assert len({i[0] for i in want}) > 3  # members retire at several checks
+    assert got == want
+    assert all(np.array_equal(x, y) and np.isfinite(y).all() for x, y in zip(state, state_w))
