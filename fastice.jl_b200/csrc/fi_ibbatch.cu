@@ -51,7 +51,7 @@ struct fi_ib_batch {
     // the shared-launch table and what it was built from
     std::vector<fi_model *> table_models;
     std::vector<KParams> table_kp;
-    std::vector<int> table_eta, table_list, table_nblist;
+    std::vector<int> table_parity, table_eta, table_list, table_nblist;
     void *d_members = nullptr;
     size_t members_cap = 0;
     uint4 *d_items = nullptr;
@@ -129,7 +129,7 @@ bool table_current(const fi_ib_batch *b, const std::vector<fi_model *> &shared) 
         const KParams k = member_kp(m);
         if (std::memcmp(&k, &b->table_kp[q], sizeof(KParams)) != 0) return false;
         const int expect = m->kp.freeze_eta ? b->table_eta[q] : (b->table_eta[q] ^ b->epar);
-        if ((int)m->eta_swapped != expect) return false;
+        if ((int)m->eta_swapped != expect || m->parity != b->table_parity[q]) return false;
         if ((int)use_list(m, k) != b->table_list[q] || m->n_blist != b->table_nblist[q]) return false;
     }
     return true;
@@ -144,6 +144,7 @@ fi_status build_table(fi_ib_batch *b, const std::vector<fi_model *> &shared) {
     std::vector<long long> off(n);
     for (int d = 0; d < 3; d++) b->max_a[d] = b->max_c[d] = 0;
     b->table_kp.resize(n);
+    b->table_parity.resize(n);
     b->table_eta.resize(n);
     b->table_list.resize(n);
     b->table_nblist.resize(n);
@@ -160,6 +161,7 @@ fi_status build_table(fi_ib_batch *b, const std::vector<fi_model *> &shared) {
         off[q] = total;
         total += list ? m->n_blist : ib_grid_blocks(m->g, !b->f64);
         b->table_kp[q] = u.p;
+        b->table_parity[q] = m->parity;
         b->table_eta[q] = m->eta_swapped;
         b->table_list[q] = list;
         b->table_nblist[q] = m->n_blist;
