@@ -412,11 +412,11 @@ fi_status reference_iteration(fi_model *m) {
 // boundary batches: on small grids their launch cost exceeds their work.  Two
 // iterations bring η / η_next back to their roles, so a pair is captured once as a
 // CUDA graph (per starting parity of the η buffers, recaptured when the parameters
-// change) and replayed for long advances.
+// or the buffers that hold the state change) and replayed for long advances.
 template <typename T>
 fi_status reference_pairs(fi_model *m, int pairs) {
     const int e = m->eta_swapped ? 1 : 0;
-    if (!m->pair_graph[e] || std::memcmp(&m->pair_kp[e], &m->kp, sizeof(KParams)) != 0) {
+    if (!m->pair_graph[e] || m->pair_parity[e] != m->parity || std::memcmp(&m->pair_kp[e], &m->kp, sizeof(KParams)) != 0) {
         if (m->pair_graph[e]) cudaGraphExecDestroy(m->pair_graph[e]);
         m->pair_graph[e] = nullptr;
         const bool sw = m->eta_swapped;
@@ -435,10 +435,13 @@ fi_status reference_pairs(fi_model *m, int pairs) {
         cudaGraphDestroy(g);
         FI_CHECK_CUDA(ie, "graph instantiate");
         m->pair_kp[e] = m->kp;
+        m->pair_parity[e] = m->parity;
     }
+    m->ib_synced = false;  // (as in reference_iteration)
     for (int q = 0; q < pairs; q++) FI_CHECK_CUDA(cudaGraphLaunch(m->pair_graph[e], m->stream), "graph launch");
     return FI_OK;
 }
+
 // Iterations of a 2D model by launches of several each (fi_tile2d.cu): an even number of
 // launches, so that the state ends in the buffers it started in, with η_next holding the
 // viscosity of the iteration before, as after the reference's swap.

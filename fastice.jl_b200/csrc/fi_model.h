@@ -50,9 +50,11 @@ struct fi_model {
     int *d_bcount = nullptr;
     int n_blist = 0;
     // reference-shaped path: two iterations captured as a CUDA graph, one per η
-    // buffer parity at the start of the pair, with the parameters they were captured with
+    // buffer parity at the start of the pair, with the parameters and the state buffers
+    // (parity) they were captured with
     cudaGraphExec_t pair_graph[2] = {nullptr, nullptr};
     KParams pair_kp[2]{};
+    int pair_parity[2] = {0, 0};
     bool ibf_stale = true;           // the volume fractions changed since d_ibf was computed
     // Full immersed-boundary iterations since anything else wrote the state, η or
     // the volume fractions.  After one, inactive strict-interior points of P, τ, V

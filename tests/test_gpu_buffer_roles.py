@@ -1,6 +1,7 @@
-"""Launch tables name the buffers that held the state when they were made.  An odd number of
-fused sweeps leaves the state in the other buffers: what was made before is made anew, bit for
-bit the same results (no-FMA build) as models that never change buffers."""
+"""Launch tables and captured pairs of iterations name the buffers that held the state when they
+were made.  A fused sweep, or a batched one of an odd number of iterations, leaves the state in
+the other buffers: what was made before is made anew, bit for bit the same results (no-FMA
+build) as models that never change buffers."""
 import numpy as np
 import pytest
 
@@ -64,3 +65,55 @@ def test_shared_table_after_fused_sweeps():
     for m in members + plain:
         m.close()
     assert not any(bad), bad
+
+
+def test_pairs_after_fused_sweeps():
+    fi = load_fastice()
+    glen = fi.ViscoplasticRegularisation(fi.PowerLawRheology(0.01, 3), 1.0)
+    slow = fi.Relaxation(glen, 0.3)
+    n = (24, 20, 12)
+    out = []
+    for path in ("auto", "reference"):
+        m = _glacier(fi, n, 3, path=path, rheology=slow)
+        m.advance(10)            # a moving viscosity runs in place, as captured pairs
+        m.set_params(rheology=glen)
+        m.advance(9)             # two full iterations, then seven fused ones
+        m.set_params(rheology=slow)
+        m.advance(1)
+        m.advance(10)
+        m.advance(10)
+        out.append(m)
+    bad = _same(*out, F3)
+    for m in out:
+        m.close()
+    assert not bad, bad
+
+
+def test_pairs_after_a_batch():
+    fi = load_fastice()
+    wall, top = ("velocity", (0.0, 0.0)), ("traction", (0.1, -0.2))
+    g = fi.UniformGrid(origin=(0.0, 0.0), extent=(1.0, 1.25), dims=(40, 31))
+    out = []
+    for batched in (True, False):
+        m = fi.IsothermalFullStokesModel(grid=g, boundary_conditions=make_bcs(fi, ((wall, wall), (wall, top)), 2),
+                                         gravity={"x": 0.3, "y": -0.7}, rheology=fi.LinearViscousRheology(1.0),
+                                         solver_params=fi.pt_params(g), path="reference", library="strict")
+        _fill(m, F2, 5)
+        m.set_field("eta", np.ones(m.field_shape("eta")))  # the viscosity of the law: held fixed by the batch
+        m.set_field("eta_next", m.get_field("eta"))
+        m.apply_bcs()
+        m.advance(8)  # captured pairs
+        if batched:
+            with fi.BatchedStokes2D([m]) as b:
+                b.advance(7)
+        else:
+            m.advance(7)
+        m.advance(1)
+        m.advance(8)
+        m.advance(9)
+        m.advance(8)
+        out.append(m)
+    bad = _same(*out, F2)
+    for m in out:
+        m.close()
+    assert not bad, bad
