@@ -122,11 +122,39 @@ bool field_used(const fi_model *m, int f) {
 
 bool is_residual(int f) { return f >= FI_FIELD_RP && f <= FI_FIELD_RVZ; }
 
+// The second state buffer that the default path of a 2D or immersed-boundary model took if there
+// was room (alloc_second_state) goes back to the device, where an allocation that the model
+// cannot do without would fail otherwise; its iterations then run in place, with the same
+// results.  Not once a state pointer was handed out: it may point there.
+bool drop_second_state(fi_model *m) {
+    if (!m->block || m->state_ptr_out) return false;
+    cudaGetLastError();
+    for (int f = 0; f < kState && m->parity; f++)
+        if (field_used(m, f) && cudaMemcpyAsync(field_raw(m->base[f], m->esz), field_raw(m->alt[f], m->esz), (m->elems + 64) * m->esz,
+                                                cudaMemcpyDeviceToDevice, m->stream) != cudaSuccess)
+            return false;
+    if (cudaStreamSynchronize(m->stream) != cudaSuccess) return false;
+    m->parity = 0;
+    for (void *&p : m->alt) p = nullptr;
+    m->eta_alt = nullptr;
+    m->tile2d = m->ib_fused = m->ib_synced = m->alt_scratch = false;
+    cudaFree(m->block);
+    m->block = nullptr, m->block_bytes = 0;
+    return true;
+}
+// a field of the model's, if need be instead of its second state buffer or its shadow's
+cudaError_t field_alloc_for(fi_model *m, void **field_ptr, size_t esz) {
+    cudaError_t e = field_alloc(field_ptr, m->elems, esz);
+    if (e != cudaSuccess && drop_second_state(m)) e = field_alloc(field_ptr, m->elems, esz);
+    if (e != cudaSuccess && m->shadow && drop_second_state(m->shadow)) e = field_alloc(field_ptr, m->elems, esz);
+    return e;
+}
+
 fi_status ensure_residual_arrays(fi_model *m) {
     for (int f = FI_FIELD_RP; f <= FI_FIELD_RVZ; f++) {
         if (!field_used(m, f) || m->base[f]) continue;
         void *p = nullptr;
-        cudaError_t e = field_alloc(&p, m->elems, m->esz);
+        cudaError_t e = field_alloc_for(m, &p, m->esz);
         if (e != cudaSuccess) return set_error("residual field allocation failed"), FI_ERR_OOM;
         FI_CHECK_CUDA(cudaMemsetAsync(field_raw(p, m->esz), 0, (m->elems + 64) * m->esz, m->stream), "memset");
         m->base[f] = p;
@@ -194,7 +222,9 @@ fi_status upload_interior(fi_model *m, int field, const void *host) {
     if (m->stage_bytes < want) {
         if (m->d_stage) cudaFree(m->d_stage);
         m->d_stage = nullptr, m->stage_bytes = 0;
-        if (cudaMalloc(&m->d_stage, want) != cudaSuccess) return cuda_fail(cudaGetLastError(), "staging buffer");
+        if (cudaMalloc(&m->d_stage, want) != cudaSuccess &&
+            !(drop_second_state(m) && cudaMalloc(&m->d_stage, want) == cudaSuccess))
+            return cuda_fail(cudaGetLastError(), "staging buffer");
         m->stage_bytes = want;
     }
     const int per = (int)std::min<size_t>(65535, std::max<size_t>(1, m->stage_bytes / plane));  // grid.y limit
@@ -370,15 +400,25 @@ fi_status refresh_ibf(fi_model *m) {
     }
     m->n_blist = cnt;
     if (m->ib_fused) {
-        FI_CHECK_CUDA(ib_runs(m->g, m->d_ibf, &m->ib_runs, m->stream), "active columns");
-        std::vector<int4> jobs;
-        ib_make_jobs(m->ib_runs, ib_job_depth({&m->ib_runs}), 0, &jobs);
-        m->ib_gen++;
+        // (without room for the lists the iterations run in place)
+        cudaError_t e = ib_runs(m->g, m->d_ibf, &m->ib_runs, m->stream);
         if (m->d_jobs) cudaFree(m->d_jobs);
-        m->d_jobs = nullptr, m->n_jobs = (int)jobs.size();
-        if (m->n_jobs > 0) {
-            FI_CHECK_CUDA(cudaMalloc(&m->d_jobs, jobs.size() * sizeof(int4)), "jobs");
-            FI_CHECK_CUDA(cudaMemcpy(m->d_jobs, jobs.data(), jobs.size() * sizeof(int4), cudaMemcpyHostToDevice), "jobs");
+        m->d_jobs = nullptr, m->n_jobs = 0;
+        m->ib_gen++;
+        if (e == cudaSuccess) {
+            std::vector<int4> jobs;
+            ib_make_jobs(m->ib_runs, ib_job_depth({&m->ib_runs}), 0, &jobs);
+            if (!jobs.empty()) e = cudaMalloc(&m->d_jobs, jobs.size() * sizeof(int4));
+            if (e == cudaSuccess && !jobs.empty()) {
+                m->n_jobs = (int)jobs.size();
+                FI_CHECK_CUDA(cudaMemcpy(m->d_jobs, jobs.data(), jobs.size() * sizeof(int4), cudaMemcpyHostToDevice), "jobs");
+            }
+        }
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (!drop_second_state(m)) m->ib_fused = m->ib_synced = false;
+        } else {
+            FI_CHECK_CUDA(e, "active columns");
         }
     }
     // captured iteration pairs hold the old list's launch size
@@ -645,7 +685,8 @@ bool model_field_used(const fi_model *m, int f) { return field_used(m, f); }
 fi_status model_ensure_second_state(fi_model *m) {
     for (int f = 0; f < kState; f++) {
         if (!field_used(m, f) || (m->alt[f] && !m->alt_scratch)) continue;
-        if (!m->alt[f] && field_alloc(&m->alt[f], m->elems, m->esz) != cudaSuccess) {
+        if (!m->alt[f] && field_alloc(&m->alt[f], m->elems, m->esz) != cudaSuccess &&
+            !(m->shadow && drop_second_state(m->shadow) && field_alloc(&m->alt[f], m->elems, m->esz) == cudaSuccess)) {
             cudaGetLastError();
             set_error("device allocation failed (second state buffer)");
             return FI_ERR_OOM;
@@ -815,10 +856,6 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
             }
 
     const size_t bytes = m->elems * m->esz;
-    if (gr.nd == 2 && desc->path == FI_PATH_AUTO) {
-        if (fi_status s = alloc_second_state(m); s != FI_OK) return fail(s);
-        m->tile2d = true;
-    }
     for (int f = 0; f < FI_FIELD_COUNT; f++) {
         if (!field_used(m, f) || is_residual(f)) continue;
         if (field_alloc(&m->base[f], m->elems, m->esz) != cudaSuccess) {
@@ -850,12 +887,6 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
     bool away = false;  // a side whose values come from elsewhere
     for (int k = 0; k < gr.nd; k++)
         for (const fi_bc &side : desc->bc[k]) away = away || side.kind == FI_BC_PERIODIC || side.kind == FI_BC_HALO;
-    if (m->ib && desc->path == FI_PATH_AUTO && !away && alloc_second_state(m) == FI_OK) {
-        // (without room for it the model keeps the in-place iterations)
-        fi_status es = encode_maps(m);
-        if (es != FI_OK) return fail(es);
-        m->ib_fused = true;
-    }
     if (m->path == FI_PATH_FUSED) {
         m->fused_variant = fused3d_default_variant(g);
         fi_status es = encode_maps(m);
@@ -868,6 +899,13 @@ fi_status fi_model_create(const fi_model_desc *desc, fi_model **out) {
         cudaGetLastError();
         set_error("norm scratch allocation failed");
         return fail(FI_ERR_OOM);
+    }
+    // last, what the model can do without: where there is no room its iterations run in place
+    if (desc->path == FI_PATH_AUTO && (gr.nd == 2 || (m->ib && !away)) && alloc_second_state(m) == FI_OK) {
+        fi_status es = m->ib ? encode_maps(m) : FI_OK;
+        if (es != FI_OK) return fail(es);
+        m->tile2d = gr.nd == 2;
+        m->ib_fused = m->ib;
     }
     if (cudaStreamSynchronize(m->stream) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "create sync"));
     *out = m;
@@ -1135,8 +1173,10 @@ static fi_status make_shadow(fi_model *m) {
     for (int c = 0; c < d.grid.nd; c++) d.gravity.kind[c] = FI_G_FIELD;
     fi_model *s = nullptr;
     fi_status st = fi_model_create(&d, &s);
+    if (st == FI_ERR_OOM && drop_second_state(m)) st = fi_model_create(&d, &s);
     if (st != FI_OK) return st;
-    if (field_alloc(&s->fP, s->elems, s->esz) != cudaSuccess) {
+    if (field_alloc_for(s, &s->fP, s->esz) != cudaSuccess &&
+        !(drop_second_state(m) && field_alloc(&s->fP, s->elems, s->esz) == cudaSuccess)) {
         fi_model_destroy(s);
         return set_error("forcing allocation failed"), FI_ERR_OOM;
     }
@@ -1272,12 +1312,15 @@ fi_status mixed_correction_begin(fi_model *m) {
     const long long n = (long long)m->elems;
     const int nd = m->d.grid.nd;
     fi_status st;
+    // (the residual fields before the copy: making them may give the second state buffer back)
+    if ((st = ensure_residual_arrays(m)) != FI_OK) return st;
+    if ((st = refresh_ibf<double>(m)) != FI_OK) return st;
+    if ((st = model_ensure_second_state(m)) != FI_OK) return st;
     for (int q = 0; q < 6; q++)
         if (field_used(m, kTauF[q]))
             FI_CHECK_CUDA(cudaMemcpyAsync(field_raw(m->nxt(kTauF[q]), m->esz), field_raw(m->cur(kTauF[q]), m->esz),
                                           (m->elems + 64) * m->esz, cudaMemcpyDeviceToDevice, m->stream),
                           "stress copy");
-    if ((st = refresh_ibf<double>(m)) != FI_OK) return st;
     FI_CHECK_CUDA(launch_compute_tau<double>(m->g, m->kp, m->ptrs<double>(), m->ib, m->stream), "projection");
     if ((st = run_batch<double>(m, stress_batch)) != FI_OK) return st;
     if ((st = residuals_t<double>(m)) != FI_OK) return st;
@@ -1478,6 +1521,7 @@ static fi_status solve_mixed(fi_model *m, const fi_solve_opts *o, fi_solve_repor
     // then continue the FP64 iteration instead of restarting it from rest.
     int outer = 0, outer_stale = 0;
     double best_outer = 1e300;
+    if ((st = ensure_residual_arrays(m)) != FI_OK) return st;
     if ((st = model_ensure_second_state(m)) != FI_OK) return st;
     while (true) {
         if ((st = mixed_picard(m)) != FI_OK) return st;
@@ -1546,7 +1590,7 @@ fi_status fi_model_volfrac_from_levelset(fi_model *m, int32_t group, const doubl
         field_free(dpsi, sizeof(double));
         for (int c = 0; c < 8; c++) field_free(tmp[c], sizeof(double));
     };
-    if (field_alloc(&dpsi, m->elems, sizeof(double)) != cudaSuccess)
+    if (field_alloc_for(m, &dpsi, sizeof(double)) != cudaSuccess)
         return cleanup(), set_error("allocation failed"), FI_ERR_OOM;
     cudaMemsetAsync(field_raw(dpsi, sizeof(double)), 0, bytes + 64 * sizeof(double), m->stream);
     // dense halo storage (n0+3) x (n1+3) x (n2+3) -> pitched storage
@@ -1565,7 +1609,7 @@ fi_status fi_model_volfrac_from_levelset(fi_model *m, int32_t group, const doubl
         if (m->is_f64()) {
             w[c] = (double *)m->base[base + c];
         } else {
-            if (field_alloc(&tmp[c], m->elems, sizeof(double)) != cudaSuccess)
+            if (field_alloc_for(m, &tmp[c], sizeof(double)) != cudaSuccess)
                 return cleanup(), set_error("allocation failed"), FI_ERR_OOM;
             cudaMemsetAsync(field_raw(tmp[c], sizeof(double)), 0, bytes + 64 * sizeof(double), m->stream);
             w[c] = (double *)tmp[c];
