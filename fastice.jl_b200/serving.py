@@ -59,19 +59,32 @@ class SolveRequest:
         return self.finished - self.arrival if self.finished is not None else math.inf
 
 
+def _held(sizes) -> int:
+    """Device bytes of allocations of these sizes: the driver hands out pieces of 2 MB,
+    which smaller allocations share."""
+    piece, total = 2 << 20, 0
+    for b in sizes:
+        total += piece // (piece // b) if b <= piece // 2 else -(-b // piece) * piece
+    return total
+
+
 def footprint_2d(n, esz: int) -> int:
-    """Device bytes of a batched 2D member: 16 state-sized arrays (P, τ×3, V×2 in
-    two buffers, η, η_next and a third viscosity buffer, the rheology's η field), rows
-    padded to 32."""
+    """Device bytes of a batched 2D member, rows padded to 32: P, τ×3, V×2, η, η_next, the
+    rheology's η field and the staging of uploads; the second state and third viscosity
+    buffer in one block."""
     pitch = ((31 + n[0] + 3 + 31) // 32) * 32
-    return 16 * pitch * (n[1] + 3) * esz + 4096
+    a = pitch * (n[1] + 3) * esz
+    return _held([a] * 9 + [min(a, 64 << 20), 7 * a]) + 4096
 
 
 def footprint_3d_ib(n, esz: int) -> int:
-    """Device bytes of a 3D immersed-boundary model: 10 state fields in two buffers, η,
-    η_next, 16 volume fractions, 4 residual fields, rows padded to 32."""
+    """Device bytes of a 3D immersed-boundary model, rows padded to 32: 10 state fields, η,
+    η_next, 16 volume fractions, 4 residual fields, the staging of uploads and the activity
+    bytes; the second state in one block."""
     pitch = ((31 + n[0] + 3 + 31) // 32) * 32
-    return 40 * pitch * (n[1] + 3) * (n[2] + 3) * esz + (1 << 20)
+    cells = pitch * (n[1] + 3) * (n[2] + 3)
+    a = cells * esz
+    return _held([a] * 32 + [min(a, 64 << 20), cells, 10 * a]) + (1 << 20)
 
 
 def rel_measure_3d(norms: np.ndarray, rho_g_inf: float, length_z: float) -> float:

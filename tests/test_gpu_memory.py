@@ -119,3 +119,39 @@ def test_mixed_solve_without_room_beside_the_second_states():
         m.close()
     assert out[0][0] == out[1][0] and out[0][0][0]["iterations"] > 60, out[0][0]  # two corrections and more
     assert all(np.array_equal(a, b) for a, b in zip(out[0][1], out[1][1]))
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_admission_estimates_cover_what_models_hold(dtype):
+    fi = load_fastice()
+    from fastice_b200 import scenarios, serving
+    esz = 8 if dtype == "f64" else 4
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def glacier(n):
+        m = scenarios.bed_model(2, n, dtype=dtype)[0]
+        m.advance(20)
+        m.compute_residuals()
+        m.residual_norms()
+        return [m]
+
+    def planes(n):
+        ms = [scenarios.inclusion_model(s, n=n, dtype=dtype)[0] for s in range(4)]
+        with fi.BatchedStokes2D(ms) as b:
+            b.step(max_iter=100, ncheck=10, tol=1e-3, rounds=1)
+        return ms
+
+    for m in glacier(16) + planes((32, 32)):  # kernels and libraries load
+        m.close()
+    for make, n, want in [(glacier, n, serving.footprint_3d_ib((n,) * 3, esz)) for n in (32, 64, 96)] + \
+                         [(planes, n, 4 * serving.footprint_2d(n, esz)) for n in ((128, 128), (511, 500), (1200, 900))]:
+        before = free()
+        ms = make(n)
+        used = before - free()
+        for m in ms:
+            m.close()
+        # (small allocations come in pieces of 2 MB)
+        assert used <= want + (4 << 20) and want <= 1.35 * used + (4 << 20), (n, used, want)
