@@ -1663,6 +1663,10 @@ fi_status fi_model_autotune(fi_model *m, int32_t iters, int32_t *best, double *m
             if (ms) ms[v] = -1.0;  // not offered in this precision
             continue;
         }
+        if (const int u = fused3d_same_launch(v); u != v) {
+            if (ms) ms[v] = ms[u];
+            continue;
+        }
         st = fi_model_set_variant(m, v);
         if (st != FI_OK) break;
         st = fi_model_advance(m, 1);  // warm-up of this launch shape

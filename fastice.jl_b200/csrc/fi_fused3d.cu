@@ -74,8 +74,9 @@ namespace fi {
 
 namespace {
 
-// Launch shapes: tile width and height, z-block depth, cluster shape (x, y).  The
-// trim flag only marks names: every shape loads the trimmed boxes.  Shapes whose
+// Launch shapes: tile width and height, z-block depth, cluster shape (x, y).  The trim flag
+// only marks names, which callers choose by: every shape loads the trimmed boxes, and the
+// autotuner does not time the same launch twice (fused3d_same_launch).  Shapes whose
 // shared memory does not fit a CTA for a precision are not offered for it.
 // fused3d_default_variant picks a 32x8 shape by the grid; the others stay for the
 // autotuner (511^3 on one box, before the direct path for ghosts: FP64 32x8 tiles 4.37 ms,
@@ -280,6 +281,14 @@ const char *fused3d_variant_name(int v) {
 int fused3d_variant_key(int v) {
     const Variant &w = kVariants[(v < 0 || v >= kNumVariants) ? 0 : v];
     return w.tx * 1000 + w.ty;
+}
+int fused3d_same_launch(int v) {
+    const Variant &w = kVariants[v];
+    for (int u = 0; u < v; u++) {
+        const Variant &o = kVariants[u];
+        if (o.tx == w.tx && o.ty == w.ty && o.zb == w.zb && o.cx == w.cx && o.cy == w.cy) return u;
+    }
+    return v;
 }
 bool fused3d_variant_fits(int v, int esz) {
     if (v < 0 || v >= kNumVariants) return false;

@@ -218,6 +218,8 @@ int fused3d_num_variants();
 int fused3d_default_variant(const Geom &g);
 // launch shapes with the same key read through the same tensor maps
 int fused3d_variant_key(int v);
+// the first launch shape that is the same launch as v under another name, or v
+int fused3d_same_launch(int v);
 // whether launch shape v fits a CTA in precision esz (8 or 4 bytes)
 bool fused3d_variant_fits(int v, int esz);
 const char *fused3d_variant_name(int v);
