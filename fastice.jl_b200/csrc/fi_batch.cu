@@ -855,8 +855,9 @@ fi_status build_regions(fi_batch *b) {
         for (int q = 0; q < n; q++) {
             const int *c = b->models[q]->d.grid.n, side = tile2d_batch_tile(b->reg_k);
             first[q] = (int)all.size();
+            const int x0 = 1 - t2_shift(c[0], side, false), y0 = 1 - t2_shift(c[1], side, false);
             for (int y = 0; y < t2_tiles(c[1], side, false); y++)
-                for (int x = 0; x < t2_tiles(c[0], side, false); x++) all.push_back(make_int4(q, x, y, 0));
+                for (int x = 0; x < t2_tiles(c[0], side, false); x++) all.push_back(make_int4(q, x0 + x * side, y0 + y * side, 0));
             cnt[q] = (int)all.size() - first[q];
         }
         const int tot = first[n] = (int)all.size();
@@ -892,7 +893,6 @@ fi_status build_regions(fi_batch *b) {
         const BInst<T> &v = reinterpret_cast<const BInst<T> *>(b->h_inst.data())[q];
         Tile2DMember<T> &u = tab[q / kTile2DMembers].m[q % kTile2DMembers];
         u.n[0] = v.n0, u.n[1] = v.n1, u.pitch = (int)v.pitch, u.forced = v.pforce;
-        for (int d = 0; d < 2; d++) u.shift[d] = t2_shift(u.n[d], tile2d_batch_tile(b->reg_k), false);
         std::memcpy(u.bc_kind, v.bc_kind, sizeof(u.bc_kind));
         std::memcpy(u.bc_val, v.bc_val, sizeof(u.bc_val));
         u.inv_dx[0] = v.idx, u.inv_dx[1] = v.idy, u.dt_P = v.dtP;

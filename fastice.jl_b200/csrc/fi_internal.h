@@ -232,11 +232,12 @@ template <typename T>
 cudaError_t launch_tile2d(const Geom &g, const KParams &p, const Ptrs<T> &in, const Ptrs<T> &out, T *eta_prev, int shape,
                           int k, bool write_prev, cudaStream_t s);
 
-// The same for the members of a batch: work item = (member, tile x, tile y).  What the kernel
-// needs of a member; f[src] is read, f[src ^ 1] written (P, τxx, τyy, τxy, V.x, V.y); η fixed.
+// The same for the members of a batch: work item = (member, first position of the tile in x,
+// y).  What the kernel needs of a member; f[src] is read, f[src ^ 1] written (P, τxx, τyy, τxy,
+// V.x, V.y); η fixed.
 template <typename T>
 struct Tile2DMember {
-    int n[2], shift[2];  // cells; t2_shift of the tiles
+    int n[2];  // cells
     int pitch, forced, bc_kind[2][2], g_kind[2];
     T inv_dx[2], dt_P, dt_tau[3], dt_V[2], g_val[2], bc_val[2][2][2];
     const T *eta, *gx, *gy, *fP;

@@ -56,7 +56,6 @@ struct Region {
 struct TileArgs {
     int k;           // iterations of this launch
     int tx, ty;      // inner tile
-    int x0, y0;      // first position of the first region
     int write_prev;  // the last launch of an advance: also write η of the iteration before
 };
 
@@ -224,10 +223,10 @@ __device__ __forceinline__ void iterate(const KParams &p, const TConst<T> &q, co
     }
 }
 
-// one region, the one around tile (bx, by)
+// one region, the one around the tile that starts at (bx0, by0)
 template <typename T, int RX, int RY, int PY, bool GF, bool BATCH>
 __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, const TConst<T> &q, const Ptrs<T> &in,
-                                           const Ptrs<T> &out, T *eta_prev, const TileArgs &ta, int bx, int by,
+                                           const Ptrs<T> &out, T *eta_prev, const TileArgs &ta, int bx0, int by0,
                                            unsigned char *t2_smem) {
     using R = Region<T, RX, RY, PY>;
     constexpr int PW = R::PW;
@@ -237,7 +236,7 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
     const int n0 = g.n[0], n1 = g.n[1];
     // (a batch has no periodic members)
     const bool px = !BATCH && p.bc_kind[0][0] == FI_BC_PERIODIC, py = !BATCH && p.bc_kind[1][0] == FI_BC_PERIODIC;
-    const int i0 = ta.x0 + bx * ta.tx, j0 = ta.y0 + by * ta.ty;
+    const int i0 = bx0 - ta.k, j0 = by0 - ta.k;
     const int gi = i0 + x;
     const int a0 = (y0 + 1) * PW + x + 1;
     const bool edge = (!px && (i0 <= 1 || i0 + RX > n0)) || (!py && (j0 <= 1 || j0 + RY > n1));
@@ -315,7 +314,6 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- the inner tile (with the ghosts beside it) to the other buffer ----
-    const int bx0 = i0 + ta.k, by0 = j0 + ta.k;
     const auto &P = v.P, &xx = v.xx, &yy = v.yy, &xy = v.xy, &vx = v.vx, &vy = v.vy, &et = v.et;
     if (!t2_owned(gi, bx0, ta.tx, n0, px)) return;
     // periodic images of centre (c) and vertex (v) values along a dimension: 0 = none
@@ -350,9 +348,10 @@ __device__ __forceinline__ void run_region(const Geom &g, const KParams &p, cons
 
 template <typename T, int RX, int RY, int PY, int MINB, bool GF>
 __global__ void __launch_bounds__(RX *RY / PY, MINB)
-    tile2d_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, T *eta_prev, TileArgs ta) {
+    tile2d_kernel(Geom g, KParams p, TConst<T> q, Ptrs<T> in, Ptrs<T> out, T *eta_prev, TileArgs ta, int x0, int y0) {
     extern __shared__ __align__(16) unsigned char t2_smem[];
-    run_region<T, RX, RY, PY, GF, false>(g, p, q, in, out, eta_prev, ta, (int)blockIdx.x, (int)blockIdx.y, t2_smem);
+    run_region<T, RX, RY, PY, GF, false>(g, p, q, in, out, eta_prev, ta, x0 + (int)blockIdx.x * ta.tx, y0 + (int)blockIdx.y * ta.ty,
+                                              t2_smem);
 }
 
 // The regions of several models, a block each; blocks past the end of the work list leave.
@@ -401,7 +400,7 @@ __global__ void __launch_bounds__(RX *RY / PY, MINB)
     const int dst = src ^ 1;
     out.P = c.f[dst][0], out.txx = c.f[dst][1], out.tyy = c.f[dst][2], out.txy = c.f[dst][3], out.Vx = c.f[dst][4],
     out.Vy = c.f[dst][5];
-    const TileArgs ta{k, tile, tile, 1 - k - c.shift[0], 1 - k - c.shift[1], 0};
+    const TileArgs ta{k, tile, tile, 0};
     run_region<T, RX, RY, PY, GF, true>(g, p, q, in, out, nullptr, ta, d.y, d.z, t2_smem);
 }
 
@@ -419,8 +418,7 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
         attr_set[dev] = true;
     }
     const bool px = p.bc_kind[0][0] == FI_BC_PERIODIC, py = p.bc_kind[1][0] == FI_BC_PERIODIC;
-    const TileArgs ta{k, RX - 2 * k, RY - 2 * k, 1 - k - t2_shift(g.n[0], RX - 2 * k, px),
-                      1 - k - t2_shift(g.n[1], RY - 2 * k, py), write_prev ? 1 : 0};
+    const TileArgs ta{k, RX - 2 * k, RY - 2 * k, write_prev ? 1 : 0};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(t2_tiles(g.n[0], ta.tx, px), t2_tiles(g.n[1], ta.ty, py));
     cfg.blockDim = dim3(R::NT);
@@ -432,7 +430,8 @@ cudaError_t launch_region(const Geom &g, const KParams &p, const Ptrs<T> &in, co
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, g, p, make_tconst<T>(p), in, out, eta_prev, ta);
+    return cudaLaunchKernelEx(&cfg, kern, g, p, make_tconst<T>(p), in, out, eta_prev, ta, 1 - t2_shift(g.n[0], ta.tx, px),
+                              1 - t2_shift(g.n[1], ta.ty, py));
 }
 
 template <typename T, bool GF>
