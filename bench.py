@@ -43,7 +43,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 TRAFFIC_BYTES_PER_CELL = {"f64": 185.7, "f32": 93.2}
 # DRAM bytes per cell of one fused immersed-boundary sweep: dram__bytes_read.sum +
 # dram__bytes_write.sum of one ncu-captured launch of the 191^3 glacier divided by its
-# cell count (profiles/fusedib_glacier191_ncu.md); the same geometry scales to 383^3.
+# cell count (profiles/fusedib_glacier191_ncu.md).  At other sizes it is an estimate: the
+# layers cut by bed and surface, which read fractions, are a smaller share of a finer grid.
 IB_TRAFFIC_BYTES_PER_CELL = {"f64": 102.9, "f32": 55.6}
 
 
@@ -648,13 +649,14 @@ def run_glacier(args):
     traffic = tr * n * n * n if tr else None
     dram = traffic / (d0["ms_per_step"] / 1e3) / 1e9 if traffic else None
     line.update({"kernel_path": d0["path"],
-                 "gpu_launches": args.steps,  # one fused sweep per iteration
+                 "gpu_launches": args.steps,  # one fused sweep per iteration (its path is called reference)
                  "roofline": {"bound": "hbm", "achieved": d0["teff_gbs"], "peak": peak, "unit": "GB/s",
                               "frac": d0["teff_gbs"] / peak, "peak_source": peak_kind,
                               "algorithmic_bytes": A * (8 if dt0 == "f64" else 4), "traffic": traffic,
                               "dram_gbs": dram, "dram_frac": dram / peak if dram else None,
-                              "note": "achieved counts 36 passes over the whole box; dram_gbs is the measured "
-                                      "traffic per iteration over its time"},
+                              "note": "achieved counts 36 passes over the whole box; traffic is the bytes per "
+                                      "cell of an ncu capture at 191^3 times the cells (an estimate on the high "
+                                      "side at 383^3), dram_gbs that over the time of an iteration"},
                  "per_dtype": res, "clocks": clocks})
     return line
 

@@ -21,8 +21,9 @@
 // Several iterations a launch.  By default the sweeps between two checks run on overlapping
 // regions instead (fi_tile2d.cu), a launch per 64 members (their parameters are kernel
 // arguments): 48 members of 63^2-511^2 71.5 -> 42.6 us an iteration in FP32 and 90.4 -> 53.7
-// in FP64, 256 members 448 -> 279 and 632 -> 351.  What bounded the sweeps above was the issue rate and a barrier per
-// iteration and tile, at 40 % of the memory's.  A batch with a chosen tile height keeps them.
+// in FP64, 256 members 449 -> 271 and 594 -> 353.  What bounded the sweeps above was the
+// issue rate and a barrier per iteration and tile, at 40 % of the memory's.  A batch with a
+// chosen tile height keeps them.
 //
 // Checks.  Every ncheck sweeps a residual kernel evaluates r_P and r_V of every
 // active instance in FP64 arithmetic and folds per-instance maxima (bit patterns

@@ -24,11 +24,12 @@
 // the ring.  After that the code itself is the limit: beyond some 100 KB of it the warps
 // wait for instructions, so there is one body for interior and boundary columns and no
 // second one for unmasked points (FP32, 383^3: 949 us with both, 742 without).  In FP64 it is
-// registers: values spilled to local memory miss every time, as next to no L1 is left beside
-// this much shared memory (36 bytes spilled at three blocks: 2118 us, two blocks 1242).
-// Measured per iteration, in place and now: FP64 383^3 1599 -> 1066 us, 191^3 260 -> 188 us;
-// FP32 383^3 1209 -> 695 us, 191^3 215 -> 129 us; a box a quarter full of ice under rough
-// beds, FP64 383^3 1355-1645 -> 1232-1559 us, 191^3 233-265 -> 166-193 us.
+// registers and the wait for fractions: values spilled to local memory miss every time, as next
+// to no L1 is left beside this much shared memory (2118 us with 36 bytes spilled), so the loads
+// stand where they are used and three blocks fit an SM with 8 bytes spilled (see sweep_ib).
+// Measured per iteration, in place and now: FP64 383^3 1599 -> 1066-1154 us by the box, 191^3
+// 260 -> 188 us; FP32 383^3 1209 -> 695 us, 191^3 215 -> 129 us; a box a quarter full of ice
+// under rough beds, FP64 383^3 1355-1645 -> 1232-1559 us, 191^3 233-265 -> 166-193 us.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -439,9 +439,9 @@ class IsothermalImmersedBoundaryFullStokesModel(_StokesBase):
 
 class BatchedIB3D:
     """Several 3D immersed-boundary models advanced by shared launches
-    (fi_ib_batch_* in the C ABI): one iteration of every small member is eight
-    launches whatever their number, and pairs of iterations replay as a CUDA graph;
-    a member whose launch spans more than 2048 blocks advances on its own stream.
+    (fi_ib_batch_* in the C ABI): one fused sweep an iteration over all members that
+    take it; the others share eight in-place launches, whose pairs replay as a CUDA
+    graph, or advance on their own stream where a launch spans more than 2048 blocks.
     Each member's iteration is the one ``advance`` runs for it alone."""
 
     def __init__(self, models=()):
@@ -483,8 +483,9 @@ class BatchedIB3D:
 class BatchedStokes2D:
     """Many independent 2D models solved together (fi_batch_* in the C ABI).
 
-    One persistent launch per PT iteration covers the tiles of every instance
-    still iterating; checks, retirement and work-list compaction run on the
+    A launch runs several PT iterations of up to 64 instances still iterating, on
+    overlapping regions (after ``set_variant``: one iteration of all of them on a
+    persistent grid of tiles); checks, retirement and work-list compaction run on the
     device, and the check-to-check step replays as a CUDA graph.  Each member
     follows advance_iteration! of its own model (linear rheology, viscosity held
     at the member's current η).  The members stay usable as models: their state

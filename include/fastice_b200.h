@@ -105,9 +105,11 @@ typedef struct {
 
 /* kernel-path selection (fi_model_desc.path) */
 typedef enum {
-    FI_PATH_AUTO = 0,      /* fused single-pass sweep where supported, else reference-shaped
-                              (2D: several iterations per launch, same results; reported as
-                              reference-shaped) */
+    FI_PATH_AUTO = 0,      /* fused single-pass sweep where supported, else reference-shaped.
+                              2D models run several iterations per launch and
+                              immersed-boundary models a fused sweep of their own, with the
+                              same results, where there is room for a second state buffer;
+                              both are reported as reference-shaped */
     FI_PATH_REFERENCE = 1, /* reference-shaped: update_sigma, BC batch, update_V, BC batch */
     FI_PATH_FUSED = 2      /* fused sweep; FI_ERR_UNSUPPORTED if the problem is not covered */
 } fi_path;
@@ -234,8 +236,9 @@ fi_status fi_model_solve(fi_model *m, const fi_solve_opts *opts, fi_solve_report
 /* swap-free view of the model state for callers that manage device memory:
  * device pointer of a field's storage (uniform halo box, see fi_model_layout).
  * The caller may write through it at any later time, so for an immersed-boundary
- * model a pointer to P, τ or V turns off for good the iterations' skipping of
- * zeros already stored at inactive points (results are the same either way). */
+ * model a pointer to P, τ or V turns off for good the fused sweep and the in-place
+ * iterations' skipping of zeros already stored at inactive points (results are the
+ * same either way; an iteration then takes 1.4-1.6 times as long). */
 fi_status fi_model_device_ptr(fi_model *m, int32_t field, void **dptr);
 /* storage box: pitch (elements per x row, >= n0+3), rows per plane (n1+3),
  * planes (n2+3, 1 in 2D); index (i,j,k) -> i + pitch*(j + rows*k), 0 = ghost. */
@@ -243,15 +246,17 @@ fi_status fi_model_layout(const fi_model *m, size_t *pitch, size_t *rows, size_t
 /* cudaStream_t of the model, as void* */
 fi_status fi_model_stream(const fi_model *m, void **stream);
 fi_status fi_model_synchronize(fi_model *m);
-/* which kernel path the model runs (fi_path, never AUTO) */
+/* which kernel path the model runs (fi_path, never AUTO): FUSED for the sweep of
+ * 3D FullStokes models; the default sweeps of 2D and immersed-boundary models count
+ * as REFERENCE, whose results they give */
 fi_status fi_model_path(const fi_model *m, int32_t *path);
 
 /* Launch shape of the fused sweep: tile width and height, z-block depth and
  * thread-block cluster shape; a model starts with one chosen by its grid.  A shape that does not
  * fit a CTA in the model's precision is rejected by fi_model_set_variant with
- * FI_ERR_UNSUPPORTED.  fi_model_autotune times every shape offered in the model's
- * precision for `iters` iterations on the model itself (so the model advances
- * like warm-up iterations), keeps the fastest and writes its index and the
+ * FI_ERR_UNSUPPORTED.  fi_model_autotune times every launch offered in the model's
+ * precision (shapes that differ in name only share a time) for `iters` iterations on
+ * the model itself (so the model advances like warm-up iterations), keeps the fastest and writes its index and the
  * per-variant milliseconds per iteration to best / ms (-1 for shapes not offered;
  * ms may be NULL, else it needs fi_fused_variant_count() slots).  No counterpart
  * in the reference (its launch shape is fixed by Chmy's Launcher). */
@@ -374,8 +379,10 @@ fi_status fi_batch_measure(fi_batch *b, double *out);
  * solve applied to the batch; no counterpart in the reference. */
 fi_status fi_batch_solve_mixed(fi_batch *b, const fi_batch_opts *opts, double inner_tol, fi_batch_item *items,
                                double *seconds);
-/* tile shapes of the batched sweep; autotune times each for `iters` iterations on
- * the batch itself (the members advance by (2 + iters) * count_of_variants) */
+/* tile shapes of the one-iteration batched sweep.  A batch advances several
+ * iterations per launch unless set_variant chooses one of these shapes; autotune times
+ * each for `iters` iterations on the batch itself (the members advance by
+ * (2 + iters) * count_of_variants) and leaves that choice as it was */
 int fi_batch_variant_count(void);
 const char *fi_batch_variant_name(int32_t variant);
 fi_status fi_batch_set_variant(fi_batch *b, int32_t variant);
@@ -383,15 +390,18 @@ fi_status fi_batch_autotune(fi_batch *b, int32_t iters, int32_t *best, double *m
 
 /* ---- batched 3D immersed-boundary iterations ------------------------------------
  * Several 3D immersed-boundary models (one dtype, one device, reference-shaped path)
- * advanced by shared launches: one iteration of every member is eight launches --
+ * advanced by shared launches.  Members whose next iterations are the fused sweep,
+ * whatever their size, share one launch an iteration; while one of them still has full
+ * iterations to run since its state changed, each runs as many alone.  For the others one
+ * iteration of every member is eight launches --
  * the masked update_σ! over a work list that concatenates the members' blocks (each
  * member's block list once its stored zeros hold), the stress boundary batches of
  * all members per dimension, the masked update_V!, the velocity boundary batches --
- * and pairs of iterations replay as one CUDA graph.  Each member's iteration is the
- * one fi_model_advance runs for it, so its result is the same alone or in the batch;
- * a member whose state changed runs its first two full iterations alone, and a member
- * whose launch already spans more than 2048 blocks (about two waves) always advances
- * alone on its own stream, overlapping the others.  The models
+ * and pairs of iterations replay as one CUDA graph; such a member runs its first two full
+ * iterations after a change alone, and where its launch already spans more than 2048 blocks
+ * (about two waves) it always advances alone on its own stream, overlapping the others.
+ * Each member's iteration is the one fi_model_advance runs for it, so its result is the
+ * same alone or in the batch.  The models
  * must outlive the batch; after fi_ib_batch_advance each member's stream is ordered
  * after the shared launches.  No counterpart in the reference, which runs one model
  * per driver loop (scripts_future_API/tm_stokes_chmy.jl:283-305). */

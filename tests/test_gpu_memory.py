@@ -2,6 +2,8 @@
 2D and immersed-boundary models is taken if there is room and given back where an allocation
 that the model cannot do without would fail: what fitted without it still runs, in place and
 with the same bits (no-FMA build)."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -20,6 +22,7 @@ class Fill:
     """Leaves `left` bytes of the device's memory free."""
 
     def __init__(self, left):
+        gc.collect()
         torch.cuda.empty_cache()
         free, _ = torch.cuda.mem_get_info()
         self.t = torch.empty(max(free - left, 0), dtype=torch.uint8, device="cuda")
@@ -128,6 +131,8 @@ def test_admission_estimates_cover_what_models_hold(dtype):
     esz = 8 if dtype == "f64" else 4
 
     def free():
+        gc.collect()  # (models that other tests left behind)
+        torch.cuda.empty_cache()
         torch.cuda.synchronize()
         return torch.cuda.mem_get_info()[0]
 
